@@ -40,9 +40,6 @@ struct Phase {
 
 }  // namespace
 
-// Longest run past a tile the batched index launch follows to finish a line.
-static constexpr int64_t kBatchMaxExtension = 8ll << 20;
-
 // Entries of a context's list of long lines handed to a warp each.
 static constexpr int64_t kLongItems = 1 << 16;
 
@@ -376,11 +373,13 @@ void free_tile_scratch(gpj_ctx* ctx, TileScratch* ts) {
     device_free(ctx, ts->offsets);
 }
 
-// Parameters of the standalone index kernel over tiles [tile_begin, tile_end).
-void set_tile_range(gpj::IndexParams* p, int64_t tile_begin, int64_t tile_end, int64_t avail) {
-    p->tile_begin = tile_begin;
-    p->tile_end = tile_end;
-    p->avail = avail;
+// Tile states for a build by the standalone kernel over `ntiles` tiles (one
+// epoch for all its launches).
+int set_tile_states(gpj_ctx* ctx, gpj::IndexParams* p, int64_t ntiles) {
+    const int rc = ensure_tile_state(ctx, ntiles);
+    p->tile_state = ctx->d_tile_state;
+    p->epoch = ctx->epoch;
+    return rc;
 }
 
 // Standalone index kernel CTAs per SM (the tuning's choice when it sets one
@@ -490,7 +489,8 @@ int run_index(gpj_ctx* ctx, const uint8_t* d_file, int64_t n, int num_levels, ui
             fused.tile_newlines = ts.counts;
             fused.colon = d_colon;
             fused.status = ctx->d_status;
-            rc = launch_tiles(ctx, fused);
+            rc = set_tile_states(ctx, &fused, fused.ntiles);
+            if (!rc) rc = launch_tiles(ctx, fused);
             if (!rc) rc = finish_tiles(ctx, fused, ts);
         }
         free_tile_scratch(ctx, &ts);
@@ -688,9 +688,12 @@ int index_pass(gpj_ctx* ctx, gpj_file* f, int num_levels, const FusedQueries* fq
     return GPJ_OK;
 }
 
-// Tiles copied per step of load_and_index: 2048 standalone-kernel tiles
-// (60 MiB), a whole number of the newline scan's 1024-tile blocks.
-constexpr int64_t kLoadTiles = 2048;
+// Chunks are counted in units of 30 KiB (gpj_tuning.chunk_tiles), multiples
+// of 1024 of them: a whole number of the newline scan's blocks of tiles.
+constexpr int64_t kChunkUnit = 30720;
+static_assert(1024 * kChunkUnit % (gpj::kNewlineBlockTiles * gpj::kStandaloneTileBytes) == 0, "whole scan blocks");
+// Units copied per step of load_and_index (60 MiB).
+constexpr int64_t kLoadUnits = 2048;
 
 // Queries load_and_index evaluates on each chunk's lines as soon as their
 // index is complete (bytecode uploaded; results strided by out_lines).
@@ -712,11 +715,11 @@ struct ChunkQueries {
 // again from the complete copy by run_index.
 //
 // host == nullptr: the input is already in f->d_data; chunks of
-// `chunk_tiles` tiles are indexed and queried in turn (index kernel, newline
+// `chunk_units` x 30 KiB are indexed and queried in turn (index kernel, newline
 // index, find_value on the lines the chunk completes), so find_value reads a
 // chunk's index while it is still in L2.
 int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_levels, const ChunkQueries* cq = nullptr,
-                   bool* queries_done = nullptr, int64_t chunk_tiles = kLoadTiles) {
+                   bool* queries_done = nullptr, int64_t chunk_units = kLoadUnits) {
     const int64_t n = f->n;
     const bool resident = host == nullptr;
     if (queries_done) *queries_done = false;
@@ -726,7 +729,8 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
     f->colon_valid = false;
     const double t0 = now_ms();
     GPJ_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-    const int64_t chunk_bytes = gpj::kStandaloneTileBytes * chunk_tiles;
+    const int64_t chunk_bytes = kChunkUnit * chunk_units;
+    const int64_t chunk_tiles = chunk_bytes / gpj::kStandaloneTileBytes;
     const int64_t nchunks = (n + chunk_bytes - 1) / chunk_bytes;
     int64_t lines = 0;
     if (nchunks <= 1) {
@@ -753,10 +757,12 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         p.newlines = f->d_nl;
         p.newline_cap = f->nl_cap;
         p.materialize = 1;
+        p.avail = n;
         p.colon = f->d_colon;
         f->colon_valid = true;  // the chunks' queries read it as their tiles write it
         TileScratch ts;
         rc = alloc_tile_scratch(ctx, n, &ts);
+        if (!rc) rc = set_tile_states(ctx, &p, p.ntiles);
         int64_t* d_lines = nullptr;  // [k + 1]: lines complete after chunk k
         if (!rc && cq) rc = device_alloc(ctx, &d_lines, static_cast<size_t>(nchunks + 1), "cudaMalloc(chunk lines)");
         if (!rc) {
@@ -778,7 +784,8 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         p.tile_newlines = ts.counts;
         auto launch_chunk = [&](int64_t k) -> int {
             const int64_t t0 = k * chunk_tiles, t1 = std::min(p.ntiles, (k + 1) * chunk_tiles);
-            set_tile_range(&p, t0, t1, resident ? n : std::min(n, (k + 2) * chunk_bytes));
+            p.tile_begin = t0;
+            p.tile_end = t1;
             if (!resident)
                 GPJ_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->chunk_events[std::min(k + 1, nchunks - 1)], 0));
             int r = launch_tiles(ctx, p);
@@ -865,7 +872,7 @@ int index_and_query(gpj_ctx* ctx, gpj_file* f, int num_levels, int nq, const uin
                                          std::to_string(num_levels));
     const int64_t chunk_tiles = ctx->tuning.chunk_tiles;
     if (!ctx->fuse_queries && chunk_tiles > 0 && !f->exact_only &&
-        f->n > gpj::kStandaloneTileBytes * chunk_tiles) {
+        f->n > kChunkUnit * chunk_tiles) {
         // chunk by chunk: index kernel, newline index, find_value on the
         // lines the chunk completes
         ChunkQueries cq;
@@ -1819,7 +1826,8 @@ int batch_index(gpj_ctx* ctx, std::vector<gpj_batch::FileRun>& files) {
         unsigned long long* status = nullptr;
         gpj::TileFile* d_tf = nullptr;
         gpj::LineFile* d_lf = nullptr;
-        rc = device_alloc(ctx, &bits, static_cast<size_t>(total_words), "cudaMalloc(batch newline bitmaps)");
+        rc = ensure_tile_state(ctx, total_tiles);
+        if (!rc) rc = device_alloc(ctx, &bits, static_cast<size_t>(total_words), "cudaMalloc(batch newline bitmaps)");
         if (!rc) rc = device_alloc(ctx, &counts, static_cast<size_t>(total_tiles), "cudaMalloc(batch tile counts)");
         if (!rc)
             rc = device_alloc(ctx, &offsets, static_cast<size_t>(gpj::newline_offsets_words(total_tiles)),
@@ -1853,22 +1861,20 @@ int batch_index(gpj_ctx* ctx, std::vector<gpj_batch::FileRun>& files) {
                 p.tile_end = total_tiles;
                 p.batch = d_tf;
                 p.batch_files = nb;
-                // a file of a batch is small (its long lines cost one CTA
-                // little) and its re-indexing alone would cost a launch
-                // and a wait: lines up to 8 MiB past a tile stay in the launch
-                p.max_extension = kBatchMaxExtension;
                 p.status = ctx->d_status;
                 p.tile_newlines = counts;
                 const int occ = tile_ctas_per_sm(ctx, levels);
                 const int64_t grid = std::min<int64_t>(total_tiles, static_cast<int64_t>(ctx->sms) * occ);
                 p.tile_counter = tile_claims(ctx);
+                p.tile_state = ctx->d_tile_state;
+                p.epoch = ctx->epoch;
                 e = cudaMemsetAsync(p.tile_counter, 0, sizeof(unsigned int), ctx->stream);
                 if (e == cudaSuccess) e = gpj::launch_tile_index_kernel(p, static_cast<int>(grid), ctx->stream);
                 ctx->launches++;
             }
             if (e == cudaSuccess) {
                 const int64_t grid = std::min<int64_t>((total_tiles + 7) / 8, static_cast<int64_t>(ctx->sms) * 8);
-                e = gpj::launch_newline_index_batch(counts, total_tiles, d_lf, nb, offsets, static_cast<int>(grid),
+                e = gpj::launch_newline_index_batch(counts, ctx->d_tile_state, total_tiles, d_lf, nb, offsets, static_cast<int>(grid),
                                                     ctx->stream);
                 ctx->launches += 2;
             }

@@ -11,9 +11,11 @@ constexpr int64_t kIndexTileBytes = 16384;  // exact kernel
 // The line-parallel kernel owns 14 KiB per tile and reads 2 KiB past it, so
 // that a tile and its look-ahead are one 64-byte word per index thread.
 constexpr int64_t kLineTileBytes = 14336;
-// The standalone index kernel owns 30 KiB per tile and reads 2 KiB past it:
-// four consecutive 64-byte words per thread of a 128-thread CTA.
-constexpr int64_t kStandaloneTileBytes = 30720;
+// The standalone index kernel: one 64-byte word per thread of a 256-thread CTA.
+constexpr int64_t kStandaloneTileBytes = 16384;
+// Tiles per block of the newline index's scan.  Chunked builds cut the file
+// at multiples of 1024 x 30 KiB (gpj_tuning.chunk_tiles), two such blocks.
+constexpr int64_t kNewlineBlockTiles = 960;
 
 // The file a tile of the standalone index kernel belongs to.  A build over
 // one file uses IndexParams' own fields; a batch passes one entry per file,
@@ -42,17 +44,17 @@ struct IndexParams {
     int num_levels;
     int64_t* newlines;  // newline_cap entries
     int64_t newline_cap;
-    unsigned long long* tile_state;  // 3 * ntiles words, tagged with `epoch`
+    unsigned long long* tile_state;  // 3 words per tile, tagged with `epoch`
     unsigned int* tile_counter;      // zeroed before the launch; the exact and standalone kernels claim tiles from it
     unsigned long long* status;      // [0] line count, [1] error bits (zeroed before)
     uint32_t epoch;                  // 1..65535
     int materialize;                 // write string_index / leveled / newlines
-    // Line-parallel kernel only: this launch indexes tiles [tile_begin,
-    // tile_end) (earlier tiles were indexed by earlier launches of the same
-    // build, with the same epoch), and only bytes [0, avail) of the file may
-    // be read (the rest may still be on its way from the host; avail is n or
-    // a multiple of 64 at or past the end of the last tile's following
-    // tile).  A line that runs past `avail` is flagged kErrLongLine.
+    // This launch indexes tiles [tile_begin, tile_end) (earlier tiles were
+    // indexed by earlier launches of the same build, with the same epoch).
+    // Line-parallel kernel: only bytes [0, avail) of the file may be read; a
+    // line that runs past `avail` is flagged kErrLongLine.  The standalone
+    // kernel reads its tiles' bytes and, where a backslash run ends before
+    // them, that run.
     int64_t tile_begin;
     int64_t tile_end;
     int64_t avail;
@@ -70,10 +72,6 @@ struct IndexParams {
     // single file (wait timeouts).
     const TileFile* batch;
     int batch_files;
-    // Longest run past its tile a CTA follows to finish a line before it
-    // flags kErrLongLine (0: the kernels' default, 64 KiB).
-    int64_t max_extension;
-
     // Queries evaluated in the same pass (line-parallel kernel only; 0 = none).
     int num_queries;
     const uint8_t* bytecode;  // all queries back to back
@@ -95,28 +93,33 @@ int index_kernel_max_ctas_per_sm(int num_levels);
 cudaError_t launch_line_index_kernel(const IndexParams& p, int grid, cudaStream_t stream);
 int line_index_max_ctas_per_sm(int num_levels);
 
-// Standalone form of the line-parallel kernel for index builds without
-// in-kernel queries: the index warps alone (up to five CTAs per SM), no tile
-// depending on another; writes string index and leveled bitmaps, and
-// newline_bits + tile_newlines instead of the newline index (same error
-// flags).  launch_newline_index then builds the newline index.
+// Standalone kernel for index builds without in-kernel queries
+// (index_tiles.cu): writes string index and leveled bitmaps, and
+// newline_bits + tile_newlines instead of the newline index; flags
+// kErrIrregular where the input is not NDJSON (so does the newline index,
+// which compares the tiles' states).  launch_newline_index then builds the
+// newline index.
 cudaError_t launch_tile_index_kernel(const IndexParams& p, int grid, cudaStream_t stream);
 int tile_index_max_ctas_per_sm(int num_levels);
 
 // Newline index from newline_bits and tile_newlines (tiles of
-// kStandaloneTileBytes): offsets of the tile counts within blocks of 1024 tiles
+// kStandaloneTileBytes): offsets of the tile counts within blocks of kNewlineBlockTiles
 // and the block sums into `offsets` (newline_offsets_words(ntiles)
 // entries), then every tile's '\n' positions; writes status[0] =
-// newlines + 1 and at most newline_cap entries.  Two launches, one stream.
+// newlines + 1 and at most newline_cap entries, and flags kErrIrregular where
+// a tile did not start in the state the tile before it ended in
+// (tile_state).  Two launches, one stream.
 cudaError_t launch_newline_index(const IndexParams& p, int64_t* offsets, int grid, cudaStream_t stream);
 // The same for tiles [t0, t1) only, once every earlier tile's newline index
-// is written (t0 and, unless t1 = ntiles, t1 multiples of 1024); the number
+// is written (t0 and, unless t1 = ntiles, t1 multiples of kNewlineBlockTiles); the number
 // of lines whose both ends are then known goes to device memory
 // `lines_done` (the newlines up to tile t1 - 1, + 1 for the last line when
 // t1 = ntiles).
 cudaError_t launch_newline_index_range(const IndexParams& p, int64_t* offsets, int64_t t0, int64_t t1,
                                        int64_t* lines_done, int grid, cudaStream_t stream);
-inline int64_t newline_offsets_words(int64_t ntiles) { return ntiles + (ntiles + 1023) / 1024; }
+inline int64_t newline_offsets_words(int64_t ntiles) {
+    return ntiles + (ntiles + kNewlineBlockTiles - 1) / kNewlineBlockTiles;
+}
 
 // Where the newline index of one file of a batch goes.
 struct LineFile {
@@ -129,9 +132,10 @@ struct LineFile {
     int64_t ntiles;
 };
 
-// Newline indexes of a batch (tile_newlines of all its tiles, ascending
-// tile_begin in `files`, a device array of nfiles entries).
-cudaError_t launch_newline_index_batch(const int32_t* tile_newlines, int64_t total_tiles, const LineFile* files,
-                                       int nfiles, int64_t* offsets, int grid, cudaStream_t stream);
+// Newline indexes of a batch (tile_newlines and tile_state of all its tiles,
+// ascending tile_begin in `files`, a device array of nfiles entries).
+cudaError_t launch_newline_index_batch(const int32_t* tile_newlines, const unsigned long long* tile_state,
+                                       int64_t total_tiles, const LineFile* files, int nfiles, int64_t* offsets,
+                                       int grid, cudaStream_t stream);
 
 }  // namespace gpj

@@ -25,8 +25,7 @@
 // Each CTA is a three-stage pipeline over its tiles (tile blockIdx.x, then
 // every gridDim.x-th):
 //  * copies: 1-D TMA bulk loads of tile + look-ahead (16 KiB) into a ring
-//    of byte slots (three here; two in the standalone kernel, whose tiles'
-//    bytes nobody reads after the tile's last barrier), issued one tile ahead;
+//    of three byte slots, issued one tile ahead;
 //  * index warps (0-7, one 64-byte word of the slot per thread): classify,
 //    resolve escapes and strings, one block scan with a reset at newlines
 //    (line starts, newline counts and each word's state at once), split
@@ -379,22 +378,6 @@ __device__ __forceinline__ TileScan tile_scan(bool reset_w, int q, int d_abs, in
     return out;
 }
 
-// Issues the TMA load of [start, start + bytes) into `dst` on `bar` (one thread).
-__device__ __forceinline__ void load_slot(const uint8_t* file, int64_t start, int64_t bytes, uint8_t* dst,
-                                          uint64_t* bar) {
-    const uint32_t bulk = static_cast<uint32_t>(bytes & ~static_cast<int64_t>(15));
-    // the last bytes of a file that do not fill 16 go by plain copies, before
-    // the arrive, so the threads waiting on `bar` see them too
-    for (int64_t i = bulk; i < bytes; i++) dst[i] = file[start + i];
-    fence_proxy_async_smem();
-    if (bulk > 0) {
-        mbar_arrive_expect_tx(bar, bulk);
-        tma_load_1d(dst, file + start, bulk, bar);
-    } else {
-        mbar_arrive(bar);
-    }
-}
-
 // Loads and classifies the 64-byte word at global position `pos` straight
 // from device memory (long extensions that do not fit the slot).
 __device__ __forceinline__ ClassMasks classify_global(const uint8_t* file, int64_t n, int64_t pos) {
@@ -604,24 +587,6 @@ __device__ int64_t find_line_end(const TileFile& p, int64_t from, int64_t tile_e
     return found == kNone ? p.n : found;
 }
 
-// The file of (batch-wide) tile t.
-__device__ __forceinline__ void fetch_tile_file(const IndexParams& p, int64_t t, TileFile* out) {
-    if (p.batch_files == 0) {
-        *out = TileFile{p.file,     p.n,     p.avail,        p.string_index, p.leveled,
-                        p.level_size, p.newline_bits, p.status, 0, p.colon};
-        return;
-    }
-    int lo = 0, hi = p.batch_files - 1;  // last file with tile_begin <= t
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (p.batch[mid].tile_begin <= t)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    *out = p.batch[lo];
-}
-
 // Starts the TMA copy of tile t into byte slot `slot` (one thread); the
 // tile's file goes into sh.desc[dslot] before the copy's mbarrier arrive, so
 // the threads that wait for the copy also see it.
@@ -779,7 +744,7 @@ __device__ void index_warps(const IndexParams& p, FShared<LV>& sh) {
                 const int esc_in = sh.carry_esc;
                 if (tid < 32) {
                     const int64_t e2 =
-                        find_line_end(F, loaded_end, tile_end, p.max_extension > 0 ? p.max_extension : kMaxExtension);
+                        find_line_end(F, loaded_end, tile_end, kMaxExtension);
                     if (tid == 0) sh.long_b = e2;
                 }
                 group_sync(kBarIndex, kIndexThreads);
@@ -964,461 +929,6 @@ __global__ void __launch_bounds__(kThreads, 2) line_index_kernel(IndexParams p) 
         line_warps<LV>(p, sh);
 }
 
-// ---- standalone index kernel ---------------------------------------------
-// Index builds without in-kernel queries (the default): 128 threads, each
-// owning four consecutive 64-byte words (256 bytes) of a 32 KiB slot, which
-// holds a 30 KiB tile and its 2 KiB look-ahead.  A thread classifies its
-// words one after another and composes their effect on the scan state
-// (string state, level, newline count) itself, so the warp scan, the
-// cross-warp scan and the tile's bookkeeping are paid once per four words.
-// What a word's classification leaves for the second pass (its masks and
-// level changes) is kept in shared memory where the word's bytes were, so
-// the slot holds bytes, then masks, then the level split's inputs and (up
-// to four levels) the level masks, and six CTAs fit per SM.  The level split deals the warp's words that hold
-// bracket cuts over its lanes (deal_levels).  Writes the string index, the ':'
-// bitmap, the leveled bitmaps and the '\n' bitmap with one 32-byte store per
-// thread and bitmap where all four words are its own, and every tile's
-// newline count; no tile waits for another.  Ownership of words and lines
-// is the line kernel's (see the top of this file), with tiles of
-// kStandaloneTileBytes.
-constexpr int kWThreads = 128;
-constexpr int kWWarps = kWThreads / 32;
-constexpr int kWK = 4;                                     // consecutive words per thread
-constexpr int kWLaneBytes = 64 * kWK;                      // 256
-constexpr int64_t kWSlot = kWThreads * kWLaneBytes;        // 32 KiB
-constexpr int64_t kWTile = kStandaloneTileBytes;           // 30 KiB
-constexpr int kWTileLanes = static_cast<int>(kWTile / kWLaneBytes);  // threads 0..119: the tile
-constexpr int kWSlotWords = static_cast<int>(kWSlot / 64);           // 512
-constexpr int64_t kWRound = kWThreads * 64;                // extension rounds: one word per thread
-static_assert(kWTile % kWLaneBytes == 0 && kWSlot - kWTile == kExtBytes, "tile + 2 KiB look-ahead per slot");
-
-// With at most four levels a word's level masks go into cells 0-3 of the
-// word itself (word_cell) once the level split has read them; with more
-// they need an array of their own, which lowers the CTAs per SM.
-template <int LV>
-constexpr bool kCellLevels = LV <= 4;
-
-template <int LV>
-struct WShared {
-    // the tile's bytes (TMA destination); after a word is classified, its
-    // 64 bytes hold eight 8-byte cells of its state (word_cell)
-    uint8_t bytes[kWSlot];
-    union {
-        // level masks, at i * kWThreads + thread (deal_levels); unused with kCellLevels
-        uint64_t acc[kCellLevels<LV> ? 1 : LV][kCellLevels<LV> ? 1 : kWSlotWords];
-        uint64_t lvacc[kWWarps][LV][32];  // split_levels_warp in the extension rounds
-    };
-    TileFile desc[2];  // the file of tile k in desc[k & 1]
-    uint64_t full;     // the slot's TMA barrier (phase k & 1 for tile k)
-    Span span_scratch[kWWarps];
-    WarpSum rscan[2][kWWarps];
-    int carry_esc;
-    int64_t long_b;
-    int64_t next_tile;  // the tile claimed for the next round
-};
-
-// Cell c (0..7) of word i of thread g, in the bytes the word was loaded
-// into.  Cells are rotated by the thread so that the threads of a warp
-// spread over the banks.  First pass: 0 quote prefix XOR, 1 '{['
-// (outside strings or not), 2 '}]', 3 structural, 4 ':', 5 '\n', 6 level
-// changes entered outside / inside a string, 7 quote parity or the string
-// state after a reset.  Second pass: 0 opening brackets, 1 closing
-// brackets, 2 structural bytes, 3 level at the word's first byte, all of
-// the word's own and outside strings; 4 string mask, 5 '\n' as before,
-// 6 ':' outside strings.  With kCellLevels, cells 0-3 then hold the masks
-// of levels 0-3: written in the second pass for a word without bracket
-// cuts, by deal_levels for a word with some.
-__device__ __forceinline__ uint64_t* word_cell(uint8_t* slot, int g, int i, int c) {
-    return reinterpret_cast<uint64_t*>(slot + kWLaneBytes * g + 64 * i + 8 * ((c + g) & 7));
-}
-
-// One 32-byte store of four words where all four are to be written and the
-// destination is 32-byte aligned, else one store per word of `mask`.
-__device__ __forceinline__ void store_words4(uint64_t* dst, const uint64_t (&v)[4], unsigned mask) {
-    if (mask == 0xFu && (reinterpret_cast<uintptr_t>(dst) & 31) == 0) {
-        asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(dst), "l"(v[0]), "l"(v[1]), "l"(v[2]),
-                     "l"(v[3])
-                     : "memory");
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-            if ((mask >> i) & 1u) dst[i] = v[i];
-    }
-}
-
-// Starts the TMA copy of tile t into the slot (one thread); its file goes
-// into desc[dslot] before the copy's arrive.
-template <int LV>
-__device__ __forceinline__ void start_wide_tile(const IndexParams& p, WShared<LV>& sh, int64_t t, int dslot) {
-    TileFile& F = sh.desc[dslot];
-    fetch_tile_file(p, t, &F);
-    const int64_t start = (t - F.tile_begin) * kWTile;
-    load_slot(F.file, start, F.avail - start < kWSlot ? F.avail - start : kWSlot, sh.bytes, &sh.full);
-}
-
-// The level split of the warp's words that hold bracket cuts (inputs in
-// cells 0-3 of each word; the other words' level masks are already in
-// place, sh.acc or their cells 0-3): such words are dealt out over the 32 lanes, one per lane per
-// pass, and each is split by split_levels, which walks its cuts.  A
-// quarter of the words have cuts and their counts differ a lot (tweets: 0.87
-// per word on average, many with eight or more), so dealing them over the
-// warp keeps most lanes busy, where a loop per thread would run as long as
-// the warp's densest thread.  `cmask`: which of the thread's four words have
-// cuts.
-template <int LV>
-__device__ __forceinline__ void deal_levels(WShared<LV>& sh, unsigned cmask) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int m = __popc(cmask);
-    int incl = m;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int o = __shfl_up_sync(~0u, incl, off);
-        if (lane >= off) incl += o;
-    }
-    const int base = incl - m;
-    const int total = __shfl_sync(~0u, incl, 31);
-    __syncwarp();
-    for (int r = 0; r < total; r += 32) {
-        const int g = r + lane;  // this lane's word with cuts, numbered across the warp
-        int o = 0;               // its thread: the last lane whose first number is <= g
-#pragma unroll
-        for (int s = 16; s > 0; s >>= 1)
-            if (__shfl_sync(~0u, base, o + s) <= g) o += s;
-        const unsigned cm = __shfl_sync(~0u, cmask, o);
-        int c = g - __shfl_sync(~0u, base, o);  // number within thread o
-        int wi = 0;                              // its word: the c-th set bit of cm
-#pragma unroll
-        for (int b = 0; b < kWK; b++) {
-            const int has = (cm >> b) & 1u;
-            if (has && c == 0) wi = b;
-            c -= has;
-        }
-        if (g < total) {
-            const int og = 32 * warp + o;
-            const uint64_t op = *word_cell(sh.bytes, og, wi, 0), cl = *word_cell(sh.bytes, og, wi, 1);
-            const uint64_t st = *word_cell(sh.bytes, og, wi, 2);
-            const int dd = static_cast<int>(static_cast<int64_t>(*word_cell(sh.bytes, og, wi, 3)));
-            uint64_t lv[LV];
-            split_levels<LV>(op, cl, st, dd, lv);
-#pragma unroll
-            for (int l = 0; l < LV; l++) {
-                if constexpr (kCellLevels<LV>)
-                    *word_cell(sh.bytes, og, wi, l) = lv[l];
-                else
-                    sh.acc[l][wi * kWThreads + og] = lv[l];
-            }
-        }
-    }
-    __syncwarp();
-}
-
-// A line that runs past the slot: the rest of it, up to its '\n', from
-// device memory, one word per thread per round (the line kernel's long-line
-// path with 128 threads).  s_in / d_in: the scan state after the slot.
-template <int LV>
-__device__ void extend_long_line(const IndexParams& p, const TileFile& F, WShared<LV>& sh, int64_t loaded_end,
-                                 int64_t tile_end, int s_in, int64_t d_in) {
-    const int tid = threadIdx.x;
-    if (tid < 32) {
-        const int64_t e2 =
-            find_line_end(F, loaded_end, tile_end, p.max_extension > 0 ? p.max_extension : kMaxExtension);
-        if (tid == 0) {
-            sh.long_b = e2;
-            // the escape state at loaded_end: the backslash run before it
-            // lies in the line, which starts in this tile with a '\n'
-            int run = 0;
-            for (int64_t j = loaded_end - 1; j >= 0 && F.file[j] == '\\'; --j) ++run;
-            sh.carry_esc = run & 1;
-        }
-    }
-    group_sync(kBarIndex, kWThreads);
-    const int64_t b_t = sh.long_b;
-    const int64_t own_end = (b_t + 63) & ~static_cast<int64_t>(63);
-    int s = s_in, esc = sh.carry_esc;
-    int64_t d = d_in;
-    for (int64_t cs = loaded_end; cs < own_end && cs < F.n; cs += kWRound) {
-        const int64_t cw = cs + 64 * tid;
-        const uint64_t cvalid = cw < own_end ? bits_between(0, F.n - cw) : 0ull;
-        ClassMasks c{0, 0, 0, 0, 0, 0, 0};
-        if (cvalid) {
-            c = classify_global(F.file, F.n, cw);
-            restrict_masks(c, cvalid);
-        }
-        // escape carry: previous word's trailing run, else the bytes before
-        const bool all_bs = c.backslash == ~0ull;
-        const int trail_par = all_bs ? 0 : (clz64(~c.backslash) & 1);
-        const int prev_par = __shfl_up_sync(~0u, trail_par, 1);
-        const int prev_all = __shfl_up_sync(~0u, all_bs ? 1 : 0, 1);
-        uint32_t ccin;
-        if ((tid & 31) > 0 && !prev_all) {
-            ccin = static_cast<uint32_t>(prev_par);
-        } else if (!cvalid) {
-            ccin = 0;  // a word past the line's end: never scan bytes past the file
-        } else {
-            int run = 0;
-            int64_t j = cw - 1;
-            while (j >= cs && __ldg(F.file + j) == '\\') {
-                ++run;
-                --j;
-            }
-            ccin = static_cast<uint32_t>((run & 1) ^ (j < cs ? esc : 0));
-        }
-        uint32_t ccout;
-        const uint64_t cesc = escaped_mask(c.backslash, ccin, &ccout);
-        const uint64_t cq = c.quote & ~cesc;
-        const uint64_t cp0 = prefix_xor(cq);
-        const Span csp{popc64(cq) & 1, popc64(c.open & ~cp0) - popc64(c.close & ~cp0), popc64(c.open) - popc64(c.close),
-                       0};
-        Span ctotal;
-        const Span cex = index_scan_span<kWWarps>(csp, sh.span_scratch, &ctotal);
-        const uint64_t ccheck = (b_t >= cw && b_t < cw + 64) ? (c.newline & (1ull << (b_t - cw))) : 0ull;
-        finish_word<LV, false>(p, F, sh, 0, c, cp0, s ^ cex.q, d + (s ? (cex.ddt - cex.dd0) : cex.dd0), cw >> 6, true,
-                               -1, cvalid, ccheck, cvalid != 0);
-        if (tid == kWThreads - 1) sh.carry_esc = static_cast<int>(ccout);
-        group_sync(kBarIndex, kWThreads);
-        esc = sh.carry_esc;
-        d += s ? (ctotal.ddt - ctotal.dd0) : ctotal.dd0;
-        s ^= ctotal.q;
-        group_sync(kBarIndex, kWThreads);
-    }
-}
-
-// Up to four levels: 6 CTAs per SM (about 37 KiB of shared memory each,
-// at most 85 registers a thread); more levels add the level-mask array.
-template <int LV>
-__global__ void __launch_bounds__(kWThreads, LV <= 4 ? 6 : (LV <= 8 ? 3 : 2)) tile_index_kernel(IndexParams p) {
-    extern __shared__ __align__(128) uint8_t smem_raw[];
-    WShared<LV>& sh = *reinterpret_cast<WShared<LV>*>(smem_raw);
-    const int tid = threadIdx.x;
-    if (tid == 0) {
-        mbar_init(&sh.full, 1);
-        fence_mbar_init();
-    }
-    // Tiles are pulled one at a time from p.tile_counter (zeroed before the
-    // launch), so a CTA that follows a long line past its tile takes fewer
-    // of them; a tile never waits for another, so any claim order is safe.
-    if (tid == 0) {
-        const int64_t t0 = p.tile_begin + static_cast<int64_t>(atomicAdd(p.tile_counter, 1u));
-        sh.next_tile = t0;
-        if (t0 < p.tile_end) start_wide_tile(p, sh, t0, 0);
-    }
-    __syncthreads();
-    int64_t k = 0;
-    for (int64_t t = sh.next_tile; t < p.tile_end; ++k) {
-        if (!mbar_wait_bounded(&sh.full, static_cast<uint32_t>(k & 1)) && tid == 0)
-            atomicOr(p.status + 1, kErrCopyTimeout);
-        uint8_t* slot = sh.bytes;
-        const TileFile& F = sh.desc[k & 1];
-        const int64_t lt = t - F.tile_begin;  // the tile's index in its file
-        const int64_t tile_start = lt * kWTile;
-        const int64_t tile_end = F.n - tile_start < kWTile ? F.n : tile_start + kWTile;
-        const int64_t loaded_end = F.avail - tile_start < kWSlot ? F.avail : tile_start + kWSlot;
-        const bool ahead = tid >= kWTileLanes;  // the thread's words lie in the look-ahead
-        const int64_t lane_start = tile_start + kWLaneBytes * tid;
-        const int64_t vend = ahead ? loaded_end : tile_end;
-
-        // ---- first pass: classify the thread's four words, compose their scan effect
-        // The escape state entering the thread's bytes: a backslash run never
-        // crosses a '\n', so inside the slot the run before them is the whole
-        // run.  Read before any thread overwrites its bytes.
-        uint32_t cin = escape_scan_back(slot, kWK * tid, 0, 0);
-        group_sync(kBarIndex, kWThreads);
-        int l_reset = 0, l_s = 0, l_dout = 0, l_din = 0, l_nl = 0;
-#pragma unroll 1
-        for (int i = 0; i < kWK; i++) {
-            const int64_t ws = lane_start + 64 * i;
-            const uint64_t valid = bits_between(0, vend - ws);
-            // the thread's words are 256 bytes apart from the next thread's,
-            // so a rotation by word would be the same for every thread
-            ClassMasks m = load_classify<false>(slot, kWK * tid + i);
-            if (valid != ~0ull) restrict_masks(m, valid);
-            uint32_t cout = 0;
-            const uint64_t esc = (m.backslash | cin) ? escaped_mask(m.backslash, cin, &cout) : 0ull;
-            cin = cout;
-            const uint64_t p0 = prefix_xor(m.quote & ~esc);
-            const bool has_nl = m.newline != 0;
-            const int f = has_nl ? ctz64(m.newline) : 0;
-            const int par_all = static_cast<int>(p0 >> 63);
-            int wq, wa, wb;
-            if (has_nl && !ahead) {
-                // a line starts after the word's first '\n': the state after the word is absolute
-                const uint64_t after = f == 63 ? 0ull : (~0ull << (f + 1));
-                const uint64_t pa = (p0 ^ (((p0 >> f) & 1ull) ? ~0ull : 0ull)) & after;
-                wq = par_all ^ static_cast<int>((p0 >> f) & 1ull);
-                wa = -1 + popc64(m.open & after & ~pa) - popc64(m.close & after & ~pa);
-                wb = 0;
-                l_reset = 1;
-                l_s = wq;
-                l_dout = wa;
-            } else {
-                wq = par_all;
-                wa = popc64(m.open & ~p0) - popc64(m.close & ~p0);  // entered outside a string
-                wb = popc64(m.open) - popc64(m.close) - wa;        // entered inside
-                if (l_reset) {
-                    l_dout += l_s ? wb : wa;
-                } else {
-                    const int a = l_dout + (l_s ? wb : wa);
-                    l_din += l_s ? wa : wb;
-                    l_dout = a;
-                }
-                l_s ^= wq;
-            }
-            l_nl += ahead ? (popc64(m.newline) << 16) : popc64(m.newline);
-            *word_cell(slot, tid, i, 0) = p0;
-            *word_cell(slot, tid, i, 1) = m.open;
-            *word_cell(slot, tid, i, 2) = m.close;
-            *word_cell(slot, tid, i, 3) = m.structural;
-            *word_cell(slot, tid, i, 4) = m.colon;
-            *word_cell(slot, tid, i, 5) = m.newline;
-            *word_cell(slot, tid, i, 6) = static_cast<uint32_t>(wa) | (static_cast<uint64_t>(static_cast<uint32_t>(wb)) << 32);
-            *word_cell(slot, tid, i, 7) = static_cast<uint64_t>(wq);
-        }
-        const TileScan sc = tile_scan<kWWarps, 64 * kWK>(l_reset != 0, l_s, l_dout, l_dout, l_din, l_nl, lt == 0,
-                                                         sh.rscan[k & 1]);
-        if (tid == 0) p.tile_newlines[t] = sc.nl_total & 0xFFFF;
-        const int ahead_nl = sc.nl_total >> 16;
-        const bool lines_here = sc.lines_here != 0;  // a line starts in this tile
-
-        // ---- second pass: final masks of the four words from the state at each one's first byte
-        int rb = sc.reset, s = sc.s, d = sc.d, nlb = sc.nl_before;
-        unsigned wmask = 0, cmask = 0;
-#pragma unroll 1
-        for (int i = 0; i < kWK; i++) {
-            const int64_t ws = lane_start + 64 * i;
-            const uint64_t valid = bits_between(0, vend - ws);
-            const uint64_t p0 = *word_cell(slot, tid, i, 0), wopen = *word_cell(slot, tid, i, 1);
-            const uint64_t wclose = *word_cell(slot, tid, i, 2), wst = *word_cell(slot, tid, i, 3);
-            const uint64_t wcolon = *word_cell(slot, tid, i, 4), nl = *word_cell(slot, tid, i, 5);
-            const uint64_t ab = *word_cell(slot, tid, i, 6);
-            const int wq = static_cast<int>(*word_cell(slot, tid, i, 7));
-            const int wa = static_cast<int32_t>(static_cast<uint32_t>(ab)), wb = static_cast<int32_t>(ab >> 32);
-            const bool has_nl = nl != 0;
-            const int f = has_nl ? ctz64(nl) : 0;
-            const uint64_t after = has_nl ? (f == 63 ? 0ull : (~0ull << (f + 1))) : ~0ull;
-            // what this CTA finishes of the word, from which state
-            bool act = false, own = true;
-            uint64_t keep = ~0ull, wp0 = p0, check = 0;
-            int s_in = s, d_in = d;
-            if (!ahead) {
-                if (rb) {
-                    // every byte of the word belongs to lines that start in this tile
-                    act = ws < tile_end;
-                    check = nl;
-                } else if (has_nl) {
-                    // the tile's first line starts after byte f of this word
-                    keep = after;
-                    act = true;
-                    own = f == 0;
-                    wp0 = (p0 ^ (((p0 >> f) & 1ull) ? ~0ull : 0ull)) & after;
-                    s_in = 0;
-                    d_in = -1;
-                    check = nl & after;
-                }
-            } else if (lines_here && (nlb >> 16) == 0 && valid) {
-                // no '\n' between the tile end and this word: the tile's last
-                // line runs into it and ends at its first '\n' (the only one checked)
-                act = !(has_nl && f == 0);
-                check = has_nl ? (1ull << f) : 0ull;
-            }
-            const uint64_t in_str = (wp0 ^ (s_in ? ~0ull : 0ull)) & valid;
-            const uint64_t open = wopen & keep & ~in_str, close = wclose & keep & ~in_str;
-            if (act && check) {
-                // every checked '\n' must be outside strings at level -1
-                if (check & in_str) atomicOr(F.status + 1, kErrIrregular);
-                for (uint64_t c = check; c; c &= c - 1) {
-                    const uint64_t below = (1ull << ctz64(c)) - 1;
-                    if (d_in + popc64(open & below) - popc64(close & below) != -1) atomicOr(F.status + 1, kErrIrregular);
-                }
-            }
-            const bool split = act && own;
-            const uint64_t sk = split ? ~0ull : 0ull;
-            const uint64_t op = open & sk, cl = close & sk, st = wst & keep & ~in_str & sk;
-            const int dd = d_in > 128 ? 128 : (d_in < -128 ? -128 : d_in);
-            const bool cut = (op | (cl << 1)) != 0;
-            // a word without bracket cuts is all at its first level (words
-            // with cuts are split by deal_levels)
-            if (kCellLevels<LV> && !cut) {
-#pragma unroll
-                for (int l = 0; l < LV; l++) *word_cell(slot, tid, i, l) = dd == l ? st : 0ull;
-            } else {
-                *word_cell(slot, tid, i, 0) = op;
-                *word_cell(slot, tid, i, 1) = cl;
-                *word_cell(slot, tid, i, 2) = st;
-                *word_cell(slot, tid, i, 3) = static_cast<uint64_t>(static_cast<int64_t>(dd));
-                if constexpr (!kCellLevels<LV>) {
-#pragma unroll
-                    for (int l = 0; l < LV; l++) sh.acc[l][i * kWThreads + tid] = dd == l ? st : 0ull;
-                }
-            }
-            *word_cell(slot, tid, i, 4) = in_str;
-            *word_cell(slot, tid, i, 6) = wcolon & keep & ~in_str;
-            cmask |= cut ? (1u << i) : 0u;
-            wmask |= split ? (1u << i) : 0u;
-            // the state at the next word's first byte
-            if (has_nl && !ahead) {
-                rb = 1;
-                s = wq;
-                d = wa;
-            } else {
-                d += s ? wb : wa;
-                s ^= wq;
-            }
-            nlb += ahead ? (popc64(nl) << 16) : popc64(nl);
-        }
-        deal_levels<LV>(sh, cmask);
-        // ---- the thread's words to the index
-        if (!ahead) {  // the '\n' bitmap of the tile's words
-            const unsigned own_nl =
-                lane_start + kWLaneBytes <= tile_end
-                    ? 0xFu
-                    : (lane_start < tile_end ? ((1u << ((tile_end - lane_start + 63) >> 6)) - 1u) : 0u);
-            if (own_nl) {
-                uint64_t v[kWK];
-#pragma unroll
-                for (int i = 0; i < kWK; i++) v[i] = *word_cell(slot, tid, i, 5);
-                store_words4(F.newline_bits + (lane_start >> 6), v, own_nl);
-            }
-        }
-        if (p.materialize && wmask) {
-            const int64_t w0 = lane_start >> 6;
-            uint64_t v[kWK];
-#pragma unroll
-            for (int i = 0; i < kWK; i++) v[i] = *word_cell(slot, tid, i, 4);
-            store_words4(F.string_index + w0, v, wmask);
-            if (F.colon) {
-#pragma unroll
-                for (int i = 0; i < kWK; i++) v[i] = *word_cell(slot, tid, i, 6);
-                store_words4(F.colon + w0, v, wmask);
-            }
-#pragma unroll
-            for (int l = 0; l < LV; l++) {
-                if (l < p.num_levels) {
-#pragma unroll
-                    for (int i = 0; i < kWK; i++) {
-                        if constexpr (kCellLevels<LV>)
-                            v[i] = *word_cell(slot, tid, i, l);
-                        else
-                            v[i] = sh.acc[l][i * kWThreads + tid];
-                    }
-                    store_words4(F.leveled + F.level_size * l + w0, v, wmask);
-                }
-            }
-        }
-        group_sync(kBarIndex, kWThreads);  // the slot and sh.acc are read: the next tile's copy may start
-        // a line past the slot is finished before the next claim, so that
-        // the tiles go to CTAs that are free
-        if (lines_here && tile_end < F.n && ahead_nl == 0 && loaded_end < F.n)
-            extend_long_line<LV>(p, F, sh, loaded_end, tile_end, sc.s_end, sc.d_end);
-        if (tid == 0) {
-            const int64_t nt = p.tile_begin + static_cast<int64_t>(atomicAdd(p.tile_counter, 1u));
-            sh.next_tile = nt;
-            if (nt < p.tile_end) start_wide_tile(p, sh, nt, static_cast<int>((k + 1) & 1));
-        }
-        group_sync(kBarIndex, kWThreads);  // the next tile's number is visible
-        t = sh.next_tile;
-    }
-}
-
 // Raises a kernel's dynamic shared memory limit, once per device (the
 // attribute belongs to the kernel's instance on the current device).
 template <class Kernel>
@@ -1433,65 +943,42 @@ cudaError_t prepare(Kernel kernel, size_t smem, std::atomic<unsigned long long>&
     return e;
 }
 
-template <int LV, bool kLines>
-struct KernelOf {
-    static void* fn() {
-        return kLines ? reinterpret_cast<void*>(line_index_kernel<LV>) : reinterpret_cast<void*>(tile_index_kernel<LV>);
-    }
-    static size_t smem() { return kLines ? sizeof(FShared<LV>) : sizeof(WShared<LV>); }
-    static int threads() { return kLines ? kThreads : kWThreads; }
-    static std::atomic<unsigned long long>& done() {
-        static std::atomic<unsigned long long> d{0};
-        return d;
-    }
-};
+template <int LV>
+std::atomic<unsigned long long>& prepared() {
+    static std::atomic<unsigned long long> d{0};
+    return d;
+}
 
-template <int LV, bool kLines>
+template <int LV>
 int occupancy() {
-    using K = KernelOf<LV, kLines>;
-    if (prepare(K::fn(), K::smem(), K::done()) != cudaSuccess) return -1;
+    if (prepare(line_index_kernel<LV>, sizeof(FShared<LV>), prepared<LV>()) != cudaSuccess) return -1;
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, K::fn(), K::threads(), K::smem()) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, line_index_kernel<LV>, kThreads, sizeof(FShared<LV>)) !=
+        cudaSuccess)
         return -1;
     return blocks;
 }
 
-template <int LV, bool kLines>
+template <int LV>
 cudaError_t launch(const IndexParams& p, int grid, cudaStream_t stream) {
-    using K = KernelOf<LV, kLines>;
-    cudaError_t e = prepare(K::fn(), K::smem(), K::done());
+    cudaError_t e = prepare(line_index_kernel<LV>, sizeof(FShared<LV>), prepared<LV>());
     if (e != cudaSuccess) return e;
-    if (kLines)
-        line_index_kernel<LV><<<grid, kThreads, sizeof(FShared<LV>), stream>>>(p);
-    else
-        tile_index_kernel<LV><<<grid, kWThreads, sizeof(WShared<LV>), stream>>>(p);
+    line_index_kernel<LV><<<grid, kThreads, sizeof(FShared<LV>), stream>>>(p);
     return cudaGetLastError();
 }
 
 }  // namespace
 
 int line_index_max_ctas_per_sm(int lv) {
-    if (lv <= 4) return occupancy<4, true>();
-    if (lv <= 8) return occupancy<8, true>();
-    return occupancy<16, true>();
+    if (lv <= 4) return occupancy<4>();
+    if (lv <= 8) return occupancy<8>();
+    return occupancy<16>();
 }
 
 cudaError_t launch_line_index_kernel(const IndexParams& p, int grid, cudaStream_t stream) {
-    if (p.num_levels <= 4) return launch<4, true>(p, grid, stream);
-    if (p.num_levels <= 8) return launch<8, true>(p, grid, stream);
-    return launch<16, true>(p, grid, stream);
-}
-
-int tile_index_max_ctas_per_sm(int lv) {
-    if (lv <= 4) return occupancy<4, false>();
-    if (lv <= 8) return occupancy<8, false>();
-    return occupancy<16, false>();
-}
-
-cudaError_t launch_tile_index_kernel(const IndexParams& p, int grid, cudaStream_t stream) {
-    if (p.num_levels <= 4) return launch<4, false>(p, grid, stream);
-    if (p.num_levels <= 8) return launch<8, false>(p, grid, stream);
-    return launch<16, false>(p, grid, stream);
+    if (p.num_levels <= 4) return launch<4>(p, grid, stream);
+    if (p.num_levels <= 8) return launch<8>(p, grid, stream);
+    return launch<16>(p, grid, stream);
 }
 
 }  // namespace gpj

@@ -3,13 +3,15 @@
 // offset of every '\n' in order; Sequential.java:14-34, built on the GPU by
 // CombinedIndex.java:117-151 with a host-side scan of per-chunk counts).
 //
-// offsets: block scans of the tile counts, 1024 tiles per CTA.  scatter: a
+// offsets: block scans of the tile counts, kNewlineBlockTiles per CTA.  scatter: a
 // warp per tile adds the sums of the earlier blocks to the tile's offset and
-// writes its positions, each lane taking consecutive bitmap words.  A batch
+// writes its positions, each lane taking consecutive bitmap words, and checks
+// that the tile started in the state the tile before it ended in.  A batch
 // of files shares one tile numbering; each file's newlines count from its
 // first tile.
 #include <cstdint>
 
+#include "device_common.cuh"
 #include "index_kernel.h"
 #include "word_ops.cuh"
 
@@ -17,12 +19,13 @@ namespace gpj {
 
 namespace {
 
-constexpr int kScanThreads = 1024;
-constexpr int kTileWordsL = static_cast<int>(kStandaloneTileBytes / 64);  // 480
-constexpr int kWordsPerLane = kTileWordsL / 32;                            // 15
+constexpr int kScanThreads = static_cast<int>(kNewlineBlockTiles);
+static_assert(kScanThreads % 32 == 0 && kScanThreads <= 1024, "one tile per thread");
+constexpr int kTileWordsL = static_cast<int>(kStandaloneTileBytes / 64);  // 256
+constexpr int kWordsPerLane = kTileWordsL / 32;                            // 8
 static_assert(kWordsPerLane * 32 == kTileWordsL, "a tile's words split evenly over a warp");
 
-// Offsets of the tile counts within blocks of 1024 tiles (coalesced, one
+// Offsets of the tile counts within blocks of kScanThreads tiles (coalesced, one
 // CTA per block, blocks blk0, blk0 + 1, ...); the block sums go after the
 // ntiles entries.
 __global__ void __launch_bounds__(kScanThreads) newline_offsets_kernel(const int32_t* counts, int64_t ntiles,
@@ -41,7 +44,7 @@ __global__ void __launch_bounds__(kScanThreads) newline_offsets_kernel(const int
     if (lane == 31) warp_total[warp] = incl;
     __syncthreads();
     int64_t before = 0, all = 0;
-#pragma unroll 8
+#pragma unroll 10
     for (int w = 0; w < kScanThreads / 32; w++) {
         if (w < warp) before += warp_total[w];
         all += warp_total[w];
@@ -71,7 +74,7 @@ __device__ __forceinline__ int64_t tiles_before(const int64_t* offsets, int64_t 
 // newline index written so far (the newlines up to t1 - 1, plus the last
 // line when t1 - 1 is the file's last tile).
 __global__ void __launch_bounds__(256) newline_scatter_kernel(const int32_t* counts, const int64_t* offsets,
-                                                              int64_t ntiles, int64_t t0, int64_t t1, LineFile one,
+                                                              const unsigned long long* states, int64_t ntiles, int64_t t0, int64_t t1, LineFile one,
                                                               const LineFile* files, int nfiles,
                                                               int64_t* lines_done) {
     const int lane = threadIdx.x & 31;
@@ -93,6 +96,10 @@ __global__ void __launch_bounds__(256) newline_scatter_kernel(const int32_t* cou
         const int64_t lt = t - F.tile_begin;
         const int64_t base = tiles_before(offsets, ntiles, t) - tiles_before(offsets, ntiles, F.tile_begin);
         if (lt == 0 && lane == 0 && F.cap > 0) F.newlines[0] = 0;
+        // the start state the tile derived from its first '\n' is the end
+        // state of the tile before it (low 48 bits; the rest is a tag)
+        if (lt > 0 && lane == 0 && ((states[3 * t + 2] ^ states[3 * (t - 1) + 1]) << 16) != 0)
+            atomicOr(F.status + 1, static_cast<unsigned long long>(kErrIrregular));
         if (lt == F.ntiles - 1 && lane == 0) F.status[0] = static_cast<unsigned long long>(base + counts[t] + 1);
         if (lines_done && t == t1 - 1 && lane == 0) *lines_done = base + counts[t] + (lt == F.ntiles - 1 ? 1 : 0);
         const int64_t w0 = lt * kTileWordsL + lane * kWordsPerLane;
@@ -124,15 +131,16 @@ __global__ void __launch_bounds__(256) newline_scatter_kernel(const int32_t* cou
 
 }  // namespace
 
-cudaError_t launch_newline_index_batch(const int32_t* tile_newlines, int64_t total_tiles, const LineFile* files,
-                                       int nfiles, int64_t* offsets, int grid, cudaStream_t stream) {
+cudaError_t launch_newline_index_batch(const int32_t* tile_newlines, const unsigned long long* tile_state,
+                                       int64_t total_tiles, const LineFile* files, int nfiles, int64_t* offsets,
+                                       int grid, cudaStream_t stream) {
     const int64_t blocks = (total_tiles + kScanThreads - 1) / kScanThreads;
     newline_offsets_kernel<<<static_cast<unsigned>(blocks), kScanThreads, 0, stream>>>(tile_newlines, total_tiles,
                                                                                        offsets, 0);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    newline_scatter_kernel<<<grid, 256, 0, stream>>>(tile_newlines, offsets, total_tiles, 0, total_tiles, LineFile{},
-                                                     files, nfiles, nullptr);
+    newline_scatter_kernel<<<grid, 256, 0, stream>>>(tile_newlines, offsets, tile_state, total_tiles, 0, total_tiles,
+                                                     LineFile{}, files, nfiles, nullptr);
     return cudaGetLastError();
 }
 
@@ -148,8 +156,8 @@ cudaError_t launch_newline_index_range(const IndexParams& p, int64_t* offsets, i
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const LineFile one{p.newline_bits, p.level_size, p.newlines, p.newline_cap, p.status, 0, ntiles};
-    newline_scatter_kernel<<<grid, 256, 0, stream>>>(p.tile_newlines, offsets, ntiles, t0, t1, one, nullptr, 0,
-                                                     lines_done);
+    newline_scatter_kernel<<<grid, 256, 0, stream>>>(p.tile_newlines, offsets, p.tile_state, ntiles, t0, t1, one,
+                                                     nullptr, 0, lines_done);
     return cudaGetLastError();
 }
 

@@ -5,6 +5,7 @@
 #include <cstdint>
 
 #include "device_common.cuh"
+#include "index_kernel.h"
 #include "word_ops.cuh"
 
 namespace gpj {
@@ -157,6 +158,40 @@ __device__ __forceinline__ int block_sum_min(int x, int64_t y, int* isum, int64_
     *total = all;
     *minimum = m;
     return before + incl - x;
+}
+
+// Issues the TMA load of [start, start + bytes) into `dst` on `bar` (one thread).
+__device__ __forceinline__ void load_slot(const uint8_t* file, int64_t start, int64_t bytes, uint8_t* dst,
+                                          uint64_t* bar) {
+    const uint32_t bulk = static_cast<uint32_t>(bytes & ~static_cast<int64_t>(15));
+    // the last bytes of a file that do not fill 16 go by plain copies, before
+    // the arrive, so the threads waiting on `bar` see them too
+    for (int64_t i = bulk; i < bytes; i++) dst[i] = file[start + i];
+    fence_proxy_async_smem();
+    if (bulk > 0) {
+        mbar_arrive_expect_tx(bar, bulk);
+        tma_load_1d(dst, file + start, bulk, bar);
+    } else {
+        mbar_arrive(bar);
+    }
+}
+
+// The file of (batch-wide) tile t.
+__device__ __forceinline__ void fetch_tile_file(const IndexParams& p, int64_t t, TileFile* out) {
+    if (p.batch_files == 0) {
+        *out = TileFile{p.file,     p.n,     p.avail,        p.string_index, p.leveled,
+                        p.level_size, p.newline_bits, p.status, 0, p.colon};
+        return;
+    }
+    int lo = 0, hi = p.batch_files - 1;  // last file with tile_begin <= t
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (p.batch[mid].tile_begin <= t)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    *out = p.batch[lo];
 }
 
 }  // namespace gpj

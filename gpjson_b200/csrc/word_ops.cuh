@@ -29,6 +29,14 @@ GPJ_HD uint32_t byte_perm(uint32_t x, uint32_t y, uint32_t s) {
 #endif
 }
 
+GPJ_HD int popc32(uint32_t x) {
+#ifdef __CUDA_ARCH__
+    return __popc(x);
+#else
+    return __builtin_popcount(x);
+#endif
+}
+
 GPJ_HD int popc64(uint64_t x) {
 #ifdef __CUDA_ARCH__
     return __popcll(x);
@@ -42,6 +50,14 @@ GPJ_HD int ctz64(uint64_t x) {  // x != 0
     return __ffsll(static_cast<long long>(x)) - 1;
 #else
     return __builtin_ctzll(x);
+#endif
+}
+
+GPJ_HD int clz32(uint32_t x) {  // x != 0
+#ifdef __CUDA_ARCH__
+    return __clz(static_cast<int>(x));
+#else
+    return __builtin_clz(x);
 #endif
 }
 
@@ -72,14 +88,17 @@ GPJ_HD uint32_t low_differs(uint32_t x, uint32_t pattern) {
 GPJ_HD uint32_t eq_bytes(uint32_t x, uint32_t pattern) { return ~(low_differs(x, pattern) | x) & 0x80808080u; }
 
 // 4x4 byte transpose of rows r0..r3: column c = {r0.b_c, r1.b_c, r2.b_c, r3.b_c}.
-GPJ_HD void transpose4(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3, uint32_t& c0,
-                       uint32_t& c1, uint32_t& c2, uint32_t& c3) {
+// kSelLow/kSelHigh of the last byte permutes put rows 0-1 first; with them
+// exchanged by kSelSwap the rows 2-3 come first (classify32).
+constexpr uint32_t kSelLow = 0x5410u, kSelHigh = 0x7632u, kSelSwap = 0x4444u;
+GPJ_HD void transpose4(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3, uint32_t& c0, uint32_t& c1, uint32_t& c2,
+                       uint32_t& c3, uint32_t sel_low = kSelLow, uint32_t sel_high = kSelHigh) {
     const uint32_t a = byte_perm(r0, r1, 0x5140), b = byte_perm(r0, r1, 0x7362);
     const uint32_t c = byte_perm(r2, r3, 0x5140), d = byte_perm(r2, r3, 0x7362);
-    c0 = byte_perm(a, c, 0x5410);
-    c1 = byte_perm(a, c, 0x7632);
-    c2 = byte_perm(b, d, 0x5410);
-    c3 = byte_perm(b, d, 0x7632);
+    c0 = byte_perm(a, c, sel_low);
+    c1 = byte_perm(a, c, sel_high);
+    c2 = byte_perm(b, d, sel_low);
+    c3 = byte_perm(b, d, sel_high);
 }
 
 // Character classes of one 64-byte word, one bit per byte.
@@ -111,11 +130,16 @@ GPJ_HD void swap_bits(uint32_t& a, uint32_t& b, int s, uint32_t m) {
 //   '"' 0x22 = 0010 0010   ':' 0x3A = 0011 1010   '\n' 0x0A = 0000 1010
 //   ',' 0x2C = 0010 1100   '\\' 0x5C = 0101 1100
 //   '[' 0x5B, '{' 0x7B = 01x1 1011 (open)   ']' 0x5D, '}' 0x7D = 01x1 1101 (close)
+//
+// `swapped`: v holds the 32 bytes with their two 16-byte halves exchanged
+// (shared-memory loads that alternate the halves between threads to spread
+// over the banks); the byte permutes put them back at no cost.
 GPJ_HD void classify32(const uint32_t v[8], uint32_t& bs, uint32_t& qt, uint32_t& nl, uint32_t& op,
-                       uint32_t& cl, uint32_t& st, uint32_t& cn) {
+                       uint32_t& cl, uint32_t& st, uint32_t& cn, bool swapped = false) {
     uint32_t r[8];
-    transpose4(v[0], v[2], v[4], v[6], r[0], r[1], r[2], r[3]);
-    transpose4(v[1], v[3], v[5], v[7], r[4], r[5], r[6], r[7]);
+    const uint32_t swap = swapped ? kSelSwap : 0u;
+    transpose4(v[0], v[2], v[4], v[6], r[0], r[1], r[2], r[3], kSelLow ^ swap, kSelHigh ^ swap);
+    transpose4(v[1], v[3], v[5], v[7], r[4], r[5], r[6], r[7], kSelLow ^ swap, kSelHigh ^ swap);
 #pragma unroll
     for (int w = 0; w < 4; w++) swap_bits(r[w], r[w + 4], 4, 0x0F0F0F0Fu);
 #pragma unroll
@@ -181,6 +205,25 @@ GPJ_HD uint64_t escaped_mask(uint64_t bs, uint32_t carry_in, uint32_t* carry_out
     return esc;
 }
 
+// escaped_mask for the bytes that are not backslashes (the others' bits are
+// not valid) with one addition: only runs starting on an even bit carry, so
+// at the byte after a run the sum's bit tells the parity of the run's start,
+// and the byte is escaped where that differs from its own bit's parity.
+GPJ_HD uint64_t escaped_bytes(uint64_t bs, uint32_t carry_in) {
+    const uint64_t kEven = 0x5555555555555555ull;
+    const uint64_t first = carry_in;
+    const uint64_t after = bs << 1;
+    const uint64_t sum = bs + (bs & ~after & kEven & ~first);
+    return (after | first) & (sum ^ kEven);
+}
+
+// Whether the word ends in an odd run of backslashes (all of them: even, 64).
+GPJ_HD bool trailing_run_odd(uint64_t bs) {
+    const uint32_t hi = ~static_cast<uint32_t>(bs >> 32), lo = ~static_cast<uint32_t>(bs);
+    const uint32_t w = hi ? hi : lo;  // 32 more do not change the parity
+    return w != 0 && (clz32(w) & 1) != 0;
+}
+
 // Inclusive prefix XOR: bit i = XOR of bits 0..i (in-string state after
 // byte i, CombinedIndex's create_string_index does the same per word).
 GPJ_HD uint64_t prefix_xor(uint64_t x) {
@@ -191,6 +234,21 @@ GPJ_HD uint64_t prefix_xor(uint64_t x) {
     x ^= x << 16;
     x ^= x << 32;
     return x;
+}
+
+// The same by 32-bit halves, three bits per step (x ^ x << s ^ x << 2 s is
+// one logic operation): 10 logic operations instead of 22.
+GPJ_HD uint32_t prefix_xor32(uint32_t x) {
+    x = x ^ (x << 1) ^ (x << 2);
+    x = x ^ (x << 3) ^ (x << 6);
+    x = x ^ (x << 9) ^ (x << 18);
+    return x ^ (x << 27);
+}
+GPJ_HD uint64_t prefix_xor_halves(uint64_t x) {
+    const uint32_t lo = prefix_xor32(static_cast<uint32_t>(x));
+    const uint32_t hi = prefix_xor32(static_cast<uint32_t>(x >> 32)) ^
+                        static_cast<uint32_t>(static_cast<int32_t>(lo) >> 31);
+    return (static_cast<uint64_t>(hi) << 32) | lo;
 }
 
 // Word summary composed across words and tiles.  Given the state before a
@@ -260,6 +318,66 @@ GPJ_HD int64_t split_levels(uint64_t open, uint64_t close, uint64_t structural, 
     for (int k = 0; k < LV; k++)
         if (d == k) lv[k] |= rest;
     return depth + popc64(open) - popc64(close);
+}
+
+// split_levels for one 32-byte half word at a cost that does not depend on
+// its brackets: the level of every byte at once as a bit-sliced running sum.
+// The change of level at each byte (+1 at an opening bracket, -1 after a
+// closing one) is held as a two's-complement number modulo 2^kPlanes, one bit
+// per plane and byte, `depth` added to the first byte's; five doubling steps
+// add the planes to themselves shifted by 1, 2, 4, 8 and 16 bytes.  With
+// LV = 2^(kPlanes - 1) levels the byte is at level k < LV where the planes
+// spell k, which is exact while every level lies in [-LV, 2 LV - 2]
+// (split_range_ok).  `at_minus_one`: the bytes at level -1.
+// The loop over cuts costs about 36 operations per cut of the warp's densest
+// word; this is 5 logic operations per step and half for four levels.
+template <int LV>
+struct SplitPlanes {
+    static_assert(LV == 4 || LV == 8 || LV == 16, "levels the index kernels are built for");
+    static constexpr int value = LV == 4 ? 3 : (LV == 8 ? 4 : 5);
+};
+
+template <int LV>
+GPJ_HD bool split_range_ok(int depth, int opens, int closes) {
+    return depth + opens < 2 * LV - 1 && depth - closes >= -LV;
+}
+
+template <int LV>
+GPJ_HD void split_half(uint32_t open, uint32_t close, uint32_t structural, int depth, uint32_t (&lv)[LV],
+                       uint32_t& at_minus_one) {
+    constexpr int P = SplitPlanes<LV>::value;
+    const uint32_t after = close << 1;  // a closing bracket counts after its byte
+    const uint32_t down = after & ~open;
+    const int first = depth + static_cast<int>(open & 1u);  // the first byte's level
+    uint32_t a[P];
+    a[0] = open ^ after;
+#pragma unroll
+    for (int i = 1; i < P; i++) a[i] = down;
+#pragma unroll
+    for (int i = 0; i < P; i++) a[i] = (a[i] & ~1u) | ((static_cast<uint32_t>(first) >> i) & 1u);
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        uint32_t carry = 0;
+#pragma unroll
+        for (int i = 0; i < P; i++) {
+            const uint32_t b = a[i] << s;
+            const uint32_t sum = a[i] ^ b ^ carry;
+            carry = (a[i] & b) | (a[i] & carry) | (b & carry);
+            a[i] = sum;
+        }
+    }
+    uint32_t ones = a[0];
+#pragma unroll
+    for (int i = 1; i < P; i++) ones &= a[i];
+    at_minus_one = ones;
+    const uint32_t in_range = structural & ~a[P - 1];
+#pragma unroll
+    for (int k = 0; k < LV; k++) {
+        uint32_t m = in_range;
+#pragma unroll
+        for (int i = 0; i < P - 1; i++) m &= (k >> i) & 1 ? a[i] : ~a[i];
+        lv[k] = m;
+    }
 }
 
 }  // namespace gpj

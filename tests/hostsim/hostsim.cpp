@@ -242,6 +242,57 @@ void hs_classify(const uint8_t* bytes, int64_t words, uint64_t* out) {
     }
 }
 
+// The same with the 16-byte halves of every 32 bytes exchanged on input.
+void hs_classify_swapped(const uint8_t* bytes, int64_t words, uint64_t* out) {
+    for (int64_t w = 0; w < words; w++) {
+        for (int h = 0; h < 2; h++) {
+            uint32_t v[8], c[7];
+            std::memcpy(v, bytes + 64 * w + 32 * h + 16, 16);
+            std::memcpy(v + 4, bytes + 64 * w + 32 * h, 16);
+            classify32(v, c[0], c[1], c[2], c[3], c[4], c[5], c[6], true);
+            for (int k = 0; k < 7; k++) out[7 * w + k] = (h ? out[7 * w + k] : 0) | static_cast<uint64_t>(c[k]) << (32 * h);
+        }
+    }
+}
+
+}  // extern "C"
+
+namespace {
+template <int LV>
+int split_word(uint64_t open, uint64_t close, uint64_t st, int depth, uint64_t* halves, uint64_t* loop,
+               uint64_t* minus_one) {
+    uint64_t lv[LV];
+    split_levels<LV>(open, close, st, depth, lv);
+    std::copy(lv, lv + LV, loop);
+    if (!split_range_ok<LV>(depth, popc64(open), popc64(close))) return 0;
+    uint32_t lo[LV], hi[LV], m_lo, m_hi;
+    const uint32_t o = static_cast<uint32_t>(open), c = static_cast<uint32_t>(close);
+    split_half<LV>(o, c, static_cast<uint32_t>(st), depth, lo, m_lo);
+    split_half<LV>(static_cast<uint32_t>(open >> 32), static_cast<uint32_t>(close >> 32),
+                   static_cast<uint32_t>(st >> 32), depth + popc32(o) - popc32(c), hi, m_hi);
+    for (int k = 0; k < LV; k++) halves[k] = static_cast<uint64_t>(hi[k]) << 32 | lo[k];
+    *minus_one = static_cast<uint64_t>(m_hi) << 32 | m_lo;
+    return 1;
+}
+}  // namespace
+
+extern "C" {
+
+// One word split by level with split_half (returns 0 where the range check
+// refuses it) and with the loop over cuts.
+int hs_split_word(int lv, uint64_t open, uint64_t close, uint64_t st, int depth, uint64_t* halves, uint64_t* loop,
+                  uint64_t* minus_one) {
+    if (lv == 4) return split_word<4>(open, close, st, depth, halves, loop, minus_one);
+    if (lv == 8) return split_word<8>(open, close, st, depth, halves, loop, minus_one);
+    return split_word<16>(open, close, st, depth, halves, loop, minus_one);
+}
+
+// The standalone index kernel's forms of the escape mask (valid off the
+// backslashes), of a word's trailing run and of the prefix XOR.
+uint64_t hs_escaped_bytes(uint64_t bs, uint32_t cin) { return escaped_bytes(bs, cin); }
+int hs_trailing_run_odd(uint64_t bs) { return trailing_run_odd(bs); }
+uint64_t hs_prefix_xor(uint64_t x, int halves) { return halves ? prefix_xor_halves(x) : prefix_xor(x); }
+
 // Escape-mask check on one word against a byte loop.
 uint64_t hs_escaped_mask(uint64_t bs, uint32_t cin, uint32_t* cout) {
     return escaped_mask(bs, cin, cout);
