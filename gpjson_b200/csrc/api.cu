@@ -40,8 +40,19 @@ struct Phase {
 
 }  // namespace
 
-// Entries of a context's list of long lines handed to a warp each.
+// Entries of a context's list of long lines handed to a warp each, and the
+// length from which they are by default (a thread walks a line's bitmaps 8
+// bytes per load, a warp 2 KiB).
 static constexpr int64_t kLongItems = 1 << 16;
+static constexpr int64_t kLongLineBytes = 8192;
+
+// Most (line, query) pairs of a file, and of a batch, that all get a warp: a
+// pair takes a warp about 9 us and a thread of the thread-per-line kernel
+// about 45, so warps win while nearly all pairs are resident at once (tweets:
+// 610 pairs 15 us against 60, 20,000 pairs 64 against 47, 59,000 pairs 160
+// against 49).
+static constexpr int64_t kFewPairs = 1 << 13;
+static constexpr int64_t kFewBatchPairs = 4096;
 
 static gpj_tuning default_tuning() {
     gpj_tuning t{};
@@ -185,6 +196,7 @@ struct gpj_batch {
         std::vector<const gpj::CompiledPath*> queries;
         int depth = 0, slots = 1;
         int64_t lines = 0;
+        bool by_warp = false;   // its lines a warp each
         size_t out_offset = 0;  // elements into `results`
     };
     std::vector<Item> items;
@@ -195,7 +207,7 @@ struct gpj_batch {
     PinnedResults* cur = nullptr;
     bool ran = false;
     // The query phase of the last run as a CUDA graph (find_value over every
-    // item, the long-line warps, the copy of the results), replayed by the
+    // item, the the copy of the results), replayed by the
     // next run when neither the requests nor the files' indexes nor the
     // launch shapes changed and no result of the last run is still held.
     struct Replay {
@@ -582,10 +594,23 @@ int query_occupancy(const gpj_ctx* ctx, int depth) {
     return want > 0 && want < occ ? want : occ;
 }
 
-// The hand-over of long lines to a warp each, or none (tuning.long_line_bytes < 0).
+// The hand-over of long lines to a warp each, or none (tuning.long_line_bytes
+// < 0).  The tuning's default stands for the library's choice.
 gpj::LongLines long_lines(const gpj_ctx* ctx) {
-    if (ctx->tuning.long_line_bytes < 0 || !ctx->d_long) return gpj::LongLines{nullptr, nullptr, 0, 0};
-    return gpj::LongLines{ctx->d_long, ctx->d_long_count, kLongItems, ctx->tuning.long_line_bytes};
+    const int64_t set = ctx->tuning.long_line_bytes;
+    if (set < 0 || !ctx->d_long) return gpj::LongLines{nullptr, nullptr, 0, 0};
+    return gpj::LongLines{ctx->d_long, ctx->d_long_count, kLongItems,
+                          set == default_tuning().long_line_bytes ? kLongLineBytes : set};
+}
+
+// Grid of a warp-per-line launch over `items` pairs (and, `listed`, an
+// unknown number of handed-over lines): a warp for each pair, so that the
+// device's own scheduling evens out lines of very different lengths.
+int warp_grid(const gpj_ctx* ctx, int64_t items, bool listed) {
+    const int64_t per_cta = gpj::kWarpThreads / 32;
+    const int64_t want = std::max<int64_t>((items + per_cta - 1) / per_cta,
+                                           listed ? static_cast<int64_t>(ctx->sms) * gpj::kListCtasPerSm : 1);
+    return static_cast<int>(std::min<int64_t>(want, 1 << 30));
 }
 
 // find_value over the file's lines, or (d_range given) over lines
@@ -614,14 +639,19 @@ int launch_query(gpj_ctx* ctx, gpj_file* f, int nq, int slots, int64_t* d_out, i
     p.newline_cap = f->nl_cap;
     p.colon = f->colon_valid ? f->d_colon : nullptr;
     p.depth = f->ir_depth;
-    p.long_lines = long_lines(ctx);
+    // (a chunk's lines are not counted yet)
+    p.by_warp = !d_range && ctx->tuning.long_line_bytes >= 0 &&
+                gpj::query_by_warp(f->num_lines, f->n, nq, kFewPairs);
+    if (!p.by_warp) p.long_lines = long_lines(ctx);
     if (p.long_lines.items)
         GPJ_CUDA(ctx, cudaMemsetAsync(ctx->d_long_count, 0, sizeof(unsigned long long), stream));
     const int64_t want =
         d_range ? INT64_MAX : (gpj::query_items(f->num_lines, nq) + gpj::kQueryThreads - 1) / gpj::kQueryThreads;
     const int64_t grid = std::max<int64_t>(
         1, std::min<int64_t>(want, static_cast<int64_t>(ctx->sms) * query_occupancy(ctx, f->ir_depth)));
-    GPJ_CUDA(ctx, gpj::launch_find_value(p, static_cast<int>(grid), ctx->sms * 2, stream));
+    GPJ_CUDA(ctx, gpj::launch_find_value(
+                      p, static_cast<int>(grid),
+                      warp_grid(ctx, p.by_warp ? f->num_lines * nq : 0, p.long_lines.items != nullptr), stream));
     ctx->launches += p.long_lines.items ? 2 : 1;
     return GPJ_OK;
 }
@@ -1989,7 +2019,7 @@ int gpj_batch_run(gpj_batch* b) {
     std::vector<uint8_t> blob;  // per file: [int32 offsets (16-byte padded)][bytecode]
     std::vector<size_t> blob_at(b->files.size());
     size_t total_out = 0;
-    int64_t total_items = 0;
+    int64_t total_items = 0, warp_items = 0, pairs = 0;
     for (size_t i = 0; i < b->files.size(); i++) {
         auto& fr = b->files[i];
         const size_t nq = fr.queries.size();
@@ -2007,8 +2037,21 @@ int gpj_batch_run(gpj_batch* b) {
         fr.lines = fr.file->num_lines;
         fr.out_offset = total_out;
         total_out += nq * static_cast<size_t>(fr.lines) * fr.slots * 2;
-        total_items += gpj::query_items(fr.lines, static_cast<int>(nq));
+        pairs += fr.lines * static_cast<int64_t>(nq);
     }
+    // Files whose lines are long, or all when the batch is small, have their
+    // lines evaluated a warp each.
+    for (auto& fr : b->files) {
+        const int nq = static_cast<int>(fr.queries.size());
+        fr.by_warp = ctx->tuning.long_line_bytes >= 0 &&
+                     (pairs <= kFewBatchPairs || gpj::query_by_warp(fr.lines, fr.file->n, nq, 0));
+        if (fr.by_warp)
+            warp_items += fr.lines * nq;
+        else
+            total_items += gpj::query_items(fr.lines, nq);
+    }
+    const int launches = (total_items > 0 ? 1 : 0) +
+                         (warp_items > 0 || (total_items > 0 && long_lines(ctx).items) ? 1 : 0);
     // what the query phase reads: replay its graph when nothing of it changed
     int depth = 0;
     for (auto& fr : b->files) depth = std::max(depth, fr.depth);
@@ -2030,7 +2073,7 @@ int gpj_batch_run(gpj_batch* b) {
         cudaError_t e = cudaGraphLaunch(b->replay.exec, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "batch query (graph)");
-        ctx->launches += long_lines(ctx).items ? 2 : 1;
+        ctx->launches += launches;
         b->cur = b->replay.dst;
         b->replays++;
         rc = end_phase(ctx, "batch_query_replay", t0);
@@ -2053,7 +2096,7 @@ int gpj_batch_run(gpj_batch* b) {
     bool captured = false;
     if (!rc) {
         std::vector<gpj::QueryFile> qf;
-        int64_t item = 0;
+        int64_t item = 0, warp_item = 0;
         for (size_t i = 0; i < b->files.size(); i++) {
             auto& fr = b->files[i];
             gpj_file* f = fr.file;
@@ -2063,8 +2106,11 @@ int gpj_batch_run(gpj_batch* b) {
                                         d_blob + blob_at[i] + header,
                                         reinterpret_cast<const int32_t*>(d_blob + blob_at[i]),
                                         static_cast<int>(nq), fr.slots, d_out + fr.out_offset, fr.lines, item,
-                                        f->colon_valid ? f->d_colon : nullptr});
-            item += gpj::query_items(fr.lines, static_cast<int>(nq));
+                                        f->colon_valid ? f->d_colon : nullptr, warp_item});
+            if (fr.by_warp)
+                warp_item += fr.lines * static_cast<int64_t>(nq);
+            else
+                item += gpj::query_items(fr.lines, static_cast<int>(nq));
         }
         cudaError_t e = cudaMemcpyAsync(d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess)
@@ -2106,15 +2152,14 @@ int gpj_batch_run(gpj_batch* b) {
         const int64_t grid = std::max<int64_t>(
             1, std::min<int64_t>((total_items + gpj::kQueryThreads - 1) / gpj::kQueryThreads,
                                  static_cast<int64_t>(ctx->sms) * query_occupancy(ctx, depth)));
-        const gpj::LongLines ll = long_lines(ctx);
         auto query_phase = [&]() -> cudaError_t {
             cudaError_t q = cudaSuccess;
-            if (total_items > 0) {
-                if (ll.items) q = cudaMemsetAsync(ctx->d_long_count, 0, sizeof(unsigned long long), ctx->stream);
-                if (q == cudaSuccess)
-                    q = gpj::launch_find_value_batch(d_qf, static_cast<int>(qf.size()), total_items, depth, ll,
-                                                     static_cast<int>(grid), ctx->sms * 2, ctx->stream);
-            }
+            const gpj::LongLines ll = total_items > 0 ? long_lines(ctx) : gpj::LongLines{};
+            if (ll.items) q = cudaMemsetAsync(ctx->d_long_count, 0, sizeof(unsigned long long), ctx->stream);
+            if (q == cudaSuccess)
+                q = gpj::launch_find_value_batch(d_qf, static_cast<int>(qf.size()), total_items, warp_items, depth, ll,
+                                                 static_cast<int>(grid), warp_grid(ctx, warp_items, ll.items != nullptr),
+                                                 ctx->stream);
             if (q == cudaSuccess && total_out > 0)
                 q = cudaMemcpyAsync(pick->p, d_out, total_out * 8, cudaMemcpyDeviceToHost, ctx->stream);
             return q;
@@ -2139,7 +2184,7 @@ int gpj_batch_run(gpj_batch* b) {
             }
             e = captured ? cudaGraphLaunch(exec, ctx->stream) : query_phase();
         }
-        ctx->launches += ll.items ? 2 : 1;
+        ctx->launches += launches;
         if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (!rc && e != cudaSuccess) rc = cuda_fail(ctx, e, "batch query");
         if (captured && !rc) {

@@ -97,19 +97,13 @@ GPJ_HD P first_of4(P w, uint64_t a, uint64_t b, uint64_t c, uint64_t d, P limit)
     return p < limit ? p : limit;
 }
 
-// `cw`/`cv`: a word of bm the caller already holds (index, value; cw = -1
-// for none), used instead of reloading it; on return they hold the word the
-// result was found in.
 template <typename P>
-GPJ_HD P next_bit(const uint64_t* bm, P from, P limit, P& cw, uint64_t& cv) {
+GPJ_HD P next_bit(const uint64_t* bm, P from, P limit) {
     if (from >= limit) return limit;
     P w = from >> 6;
     const P wend = ((limit - 1) >> 6) + 1;
-    const uint64_t first = w == cw ? cv : bm[w];
-    const uint64_t m = first & (~0ull << (from & 63));
+    const uint64_t m = bm[w] & (~0ull << (from & 63));
     if (m) {
-        cw = w;
-        cv = first;
         const P p = (w << 6) + ctz64(m);
         return p < limit ? p : limit;
     }
@@ -117,8 +111,6 @@ GPJ_HD P next_bit(const uint64_t* bm, P from, P limit, P& cw, uint64_t& cv) {
     for (++w; w < wend && w < (from >> 6) + 3; ++w) {
         const uint64_t x = bm[w];
         if (x) {
-            cw = w;
-            cv = x;
             const P p = (w << 6) + ctz64(x);
             return p < limit ? p : limit;
         }
@@ -128,61 +120,7 @@ GPJ_HD P next_bit(const uint64_t* bm, P from, P limit, P& cw, uint64_t& cv) {
         const uint64_t b = w + 1 < wend ? bm[w + 1] : 0;
         const uint64_t c = w + 2 < wend ? bm[w + 2] : 0;
         const uint64_t d = w + 3 < wend ? bm[w + 3] : 0;
-        if (a | b | c | d) {
-            const P p = first_of4<P>(w, a, b, c, d, limit);
-            cw = w + (a ? 0 : (b ? 1 : (c ? 2 : 3)));
-            cv = a ? a : (b ? b : (c ? c : d));
-            return p;
-        }
-    }
-    return limit;
-}
-
-template <typename P>
-GPJ_HD P next_bit(const uint64_t* bm, P from, P limit) {
-    P cw = -1;
-    uint64_t cv = 0;
-    return next_bit<P>(bm, from, limit, cw, cv);
-}
-
-// First position in [from, limit) set in bm and (in `filt`, or not in it
-// when `invert`), or `limit`; cw/cv as in next_bit, for the combined word
-// bm[w] & (filt[w] ^ flip).
-template <typename P>
-GPJ_HD P next_bit_filtered(const uint64_t* bm, const uint64_t* filt, bool invert, P from, P limit, P& cw,
-                           uint64_t& cv) {
-    if (from >= limit) return limit;
-    P w = from >> 6;
-    const P wend = ((limit - 1) >> 6) + 1;
-    const uint64_t flip = invert ? ~0ull : 0ull;
-    const uint64_t first = w == cw ? cv : bm[w] & (filt[w] ^ flip);
-    const uint64_t m = first & (~0ull << (from & 63));
-    if (m) {
-        cw = w;
-        cv = first;
-        const P p = (w << 6) + ctz64(m);
-        return p < limit ? p : limit;
-    }
-    for (++w; w < wend && w < (from >> 6) + 3; ++w) {
-        const uint64_t x = bm[w] & (filt[w] ^ flip);
-        if (x) {
-            cw = w;
-            cv = x;
-            const P p = (w << 6) + ctz64(x);
-            return p < limit ? p : limit;
-        }
-    }
-    for (; w < wend; w += 4) {
-        const uint64_t a = bm[w] & (filt[w] ^ flip);
-        const uint64_t b = w + 1 < wend ? bm[w + 1] & (filt[w + 1] ^ flip) : 0;
-        const uint64_t c = w + 2 < wend ? bm[w + 2] & (filt[w + 2] ^ flip) : 0;
-        const uint64_t d = w + 3 < wend ? bm[w + 3] & (filt[w + 3] ^ flip) : 0;
-        if (a | b | c | d) {
-            const P p = first_of4<P>(w, a, b, c, d, limit);
-            cw = w + (a ? 0 : (b ? 1 : (c ? 2 : 3)));
-            cv = a ? a : (b ? b : (c ? c : d));
-            return p;
-        }
+        if (a | b | c | d) return first_of4<P>(w, a, b, c, d, limit);
     }
     return limit;
 }
@@ -310,18 +248,118 @@ struct PackedLevels {
     GPJ_HD void set_idx(int k, int64_t v) { index[k * stride] = static_cast<int32_t>(v); }
 };
 
+// The key a MOVE_TO_KEY looks for, with the bytes that end right before the
+// ':' of a match in the usual layout: the key's last three bytes (its opening
+// quote among them when it is shorter) and its closing quote.
+struct Key {
+    const uint8_t* bytes;
+    int32_t len;
+    uint32_t tail, mask;  // mask 0: every candidate takes the general check
+    GPJ_HD void set(const uint8_t* b, int32_t n) {
+        bytes = b;
+        len = n;
+        mask = n == 0 || b[n - 1] == '\\' ? 0u : (n == 1 ? 0xFFFFFF00u : ~0u);
+        tail = 0x22000000u;
+        if (n >= 1) tail |= static_cast<uint32_t>(b[n - 1]) << 16;
+        if (n >= 1) tail |= static_cast<uint32_t>(n >= 2 ? b[n - 2] : '"') << 8;
+        if (n >= 2) tail |= static_cast<uint32_t>(n >= 3 ? b[n - 3] : '"');
+    }
+};
+
+// The four bytes at p, little endian (on the device two aligned loads, so
+// up to three bytes after p + 4 are read as well).
+GPJ_HD uint32_t load4(const uint8_t* p) {
+#ifdef __CUDA_ARCH__
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~static_cast<uintptr_t>(3));
+    return __funnelshift_r(w[0], w[1], 8 * (a & 3));
+#else
+    return p[0] | p[1] << 8 | p[2] << 16 | static_cast<uint32_t>(p[3]) << 24;
+#endif
+}
+
+// What a key search looks at.
+template <typename P>
+struct KeyScope {
+    const uint8_t* file;
+    P hi;  // bytes at or after it are not read
+    const uint64_t* string_index;
+    P line_start;
+};
+
+// Whether the string before the structural ':' at p is the key
+// (find_value.cu:225-251): the key's bytes end at the last in-string byte
+// before p, with a '"' before them.
+template <typename P>
+GPJ_HD bool key_at(const KeyScope<P>& v, const Key& key, P p) {
+    const int64_t start = static_cast<int64_t>(prev_bit<P>(v.string_index, p - 1, v.line_start)) - key.len;
+    if (start < v.line_start || v.file[start] != '"') return false;
+    for (int32_t k = 0; k < key.len; k++)
+        if (key.bytes[k] != v.file[start + 1 + k]) return false;
+    return true;
+}
+
+// Whether key_at can be true, from the four bytes before p alone.  A '"'
+// right before p that no backslash precedes closes a string (the ':' is
+// outside strings), so the key's last byte is at p - 2 and must be the one
+// before that '"'.  Anything else (blanks before the ':', a backslash, the
+// line's or view's edges, a key with mask 0) may be.  One four-byte
+// comparison thus rejects nearly every other key, without the string index
+// and the key's bytes one by one.
+template <typename P>
+GPJ_HD bool key_may_be_at(const KeyScope<P>& v, const Key& key, P p) {
+    if (key.mask == 0 || p - v.line_start < 4 || p + 4 > v.hi) return true;
+    const uint32_t t = load4(v.file + p - 4);
+    return ((t ^ key.tail) & key.mask) == 0 || (t & 0xFF000000u) != 0x22000000u || (t & 0x00FF0000u) == 0x005C0000u;
+}
+
 // How the interpreter scans: one thread alone (SeqScan), or the 32 lanes of
 // a warp together on one line (WarpScan, query_kernel.cu), every lane
 // holding the same interpreter state.
 struct SeqScan {
     template <typename P>
-    GPJ_HD static P next(const uint64_t* bm, P from, P limit, P& cw, uint64_t& cv) {
-        return next_bit<P>(bm, from, limit, cw, cv);
+    GPJ_HD static P next(const uint64_t* bm, P from, P limit) {
+        return next_bit<P>(bm, from, limit);
     }
+    // First structural ':' of `bits` in [from, limit) whose string is the key, or `limit`.
     template <typename P>
-    GPJ_HD static P next_filtered(const uint64_t* bm, const uint64_t* filt, bool invert, P from, P limit, P& cw,
-                                  uint64_t& cv) {
-        return next_bit_filtered<P>(bm, filt, invert, from, limit, cw, cv);
+    GPJ_HD static P find_key(const KeyScope<P>& v, const Key& key, const uint64_t* bits, const uint64_t* colon, P from,
+                             P limit) {
+        if (from >= limit) return limit;
+        P w = from >> 6;
+        const P last = (limit - 1) >> 6;
+        uint64_t x = bits[w] & (colon ? colon[w] : ~0ull) & (~0ull << (from & 63));
+        for (;;) {
+            while (x == 0) {
+                if (w == last) return limit;
+                ++w;
+                x = bits[w] & (colon ? colon[w] : ~0ull);
+            }
+            const P p = (w << 6) + ctz64(x);
+            if (p >= limit) return limit;
+            x &= x - 1;
+            if (key_may_be_at<P>(v, key, p) && (colon || v.file[p] == ':') && key_at<P>(v, key, p)) return p;
+        }
+    }
+    // Position of the `count`-th (from 1) ',' among the bytes of `bits` in [from, limit), or `limit`.
+    template <typename P>
+    GPJ_HD static P find_comma(const uint8_t* file, const uint64_t* bits, const uint64_t* colon, P from, P limit,
+                               int64_t count) {
+        if (from >= limit || count < 1) return limit;
+        P w = from >> 6;
+        const P last = (limit - 1) >> 6;
+        uint64_t x = bits[w] & (colon ? ~colon[w] : ~0ull) & (~0ull << (from & 63));
+        for (;;) {
+            while (x == 0) {
+                if (w == last) return limit;
+                ++w;
+                x = bits[w] & (colon ? ~colon[w] : ~0ull);
+            }
+            const P p = (w << 6) + ctz64(x);
+            if (p >= limit) return limit;
+            x &= x - 1;
+            if (file[p] == ',' && --count == 0) return p;
+        }
     }
     template <typename P>
     GPJ_HD static P skip(const uint8_t* file, P j, P hi) {
@@ -345,25 +383,16 @@ GPJ_HD int run_line_core(const uint8_t* file, P n, P hi, int skip_end, const uin
 
     int pc = 0, cur = 0, result_index = 0;
     stored = 0;
-    uint8_t type = 0xFF;
-    P want_len = 0;
+    Key key{};
+    const KeyScope<P> scope{file, hi, string_index, line_start};
     int64_t want_index = -1;
-    const uint8_t* want = nullptr;
-    bool execute = true;
-
     P j = line_start;
-    // the search state: j came from next_bit (so it is a structural bit of
-    // level cur), and the bitmap word next_bit found it in
-    bool found = false;
-    P cw = -1;
-    uint64_t cv = 0;
-    P cend = lv.end(cur);  // lv.end(cur), kept while searching (only opcodes change it)
-    P cidx = -1;           // lv.idx(cur) during an index search, written back at its match
+    P cend = line_end;  // lv.end(cur) once the opcodes have run
     while (j < cend && j < n) {
-        const bool ran = execute;
-        while (execute) {
-            type = ir[pc++];
-            switch (type) {
+        // The opcodes up to the next search.
+        bool to_key = false, to_index = false;
+        while (!to_key && !to_index) {
+            switch (ir[pc++]) {
                 case 0:  // END
                     return kLineDone;
                 case 1: {  // STORE_RESULT (find_value.cu:59-82)
@@ -385,19 +414,18 @@ GPJ_HD int run_line_core(const uint8_t* file, P n, P hi, int skip_end, const uin
                     ++cur;
                     if (lv.end(cur) == -1) {
                         const P lim = lv.end(cur - 1);
-                        P mw = -1;
-                        uint64_t mv = 0;
-                        const P m = Scan::template next<P>(levels + level_size * (cur - 1), j + 1, lim, mw, mv);
+                        const P m = Scan::template next<P>(levels + level_size * (cur - 1), j + 1, lim);
                         if (m < lim) lv.set_end(cur, m);
                     }
                     break;
                 }
-                case 4:  // MOVE_TO_KEY (:112-130)
-                    want_len = static_cast<P>(read_varint(ir, pc));
-                    want = ir + pc;
-                    pc += static_cast<int>(want_len);
-                    execute = false;
+                case 4: {  // MOVE_TO_KEY (:112-130)
+                    const int32_t len = static_cast<int32_t>(read_varint(ir, pc));
+                    key.set(ir + pc, len);
+                    pc += len;
+                    to_key = true;
                     break;
+                }
                 case 5:  // MOVE_TO_INDEX (:131-169)
                     want_index = read_varint(ir, pc);
                     if (lv.idx(cur) == -1) {
@@ -406,22 +434,19 @@ GPJ_HD int run_line_core(const uint8_t* file, P n, P hi, int skip_end, const uin
                         if (file[j] != '[') return kLineDone;
                         lv.set_idx(cur, 0);
                     }
-                    if (want_index == 0) {
+                    if (want_index == 0)
                         ++j;
-                        execute = true;
-                    } else {
-                        execute = false;
-                        cidx = lv.idx(cur);
-                    }
+                    else
+                        to_index = true;
                     break;
                 case 6: {  // EXPRESSION_STRING_EQUALS (:170-210)
-                    want_len = static_cast<P>(read_varint(ir, pc));
-                    want = ir + pc;
-                    pc += static_cast<int>(want_len);
+                    const P len = static_cast<P>(read_varint(ir, pc));
+                    const uint8_t* want = ir + pc;
+                    pc += static_cast<int>(len);
                     j = Scan::template skip<P>(file, j, hi);  // [bounded]
                     if (j >= hi && skip_end) return kLineDeferred;
-                    if (lv.end(cur) - j != want_len) return kLineDone;
-                    for (P k = 0; k < want_len; k++)
+                    if (lv.end(cur) - j != len) return kLineDone;
+                    for (P k = 0; k < len; k++)
                         if (want[k] != file[j + k]) return kLineDone;
                     break;
                 }
@@ -429,61 +454,21 @@ GPJ_HD int run_line_core(const uint8_t* file, P n, P hi, int skip_end, const uin
                     return kLineDone;
             }
         }
-        if (ran) cend = lv.end(cur);
-
-        // Searching: j is a candidate position ([bounded] only inside the file).
-        if (j < hi) {
-            const uint64_t* bits = levels + level_size * cur;
-            const bool structural = found || ((bits[j >> 6] >> (j & 63)) & 1u);
-            const uint8_t at = file[j];
-            if (type == 4) {  // key match at a structural ':' (:225-251)
-                // Loads that do not depend on each other are issued together:
-                // the string-index word before j, and the byte where the key's
-                // opening quote is when the key ends right before the ':'
-                // (the usual layout), checked against the real position below.
-                const uint64_t sw = j > line_start ? string_index[(j - 1) >> 6] : 0;
-                const int64_t guess = static_cast<int64_t>(j) - 2 - want_len;
-                const uint8_t at_guess = guess >= line_start ? file[guess] : 0;
-                if (structural && at == ':') {
-                    const P string_end = prev_bit<P>(string_index, sw, j - 1, line_start);
-                    const int64_t string_start = static_cast<int64_t>(string_end) - want_len;
-                    if (string_start >= line_start &&
-                        (string_start == guess ? at_guess : file[string_start]) == '"') {
-                        bool same = true;
-                        for (P k = 0; k < want_len; k++) {
-                            if (want[k] != file[string_start + k + 1]) {
-                                same = false;
-                                break;
-                            }
-                        }
-                        execute = same;
-                    }
-                }
-            } else if (type == 5) {  // index match at a structural ',' (:252-259)
-                if (structural && at == ',') {
-                    ++cidx;
-                    if (want_index == cidx) {
-                        lv.set_idx(cur, cidx);
-                        execute = true;
-                    }
-                }
-            }
-        }
-        ++j;
-        found = false;
-        if (!execute) {
-            // Nothing happens until the next structural bit of this level.
-            const P lim = cend < n ? cend : n;
-            if (j < lim) {
-                if (colon)
-                    j = Scan::template next_filtered<P>(levels + level_size * cur, colon, type != 4, j, lim, cw, cv);
-                else
-                    j = Scan::template next<P>(levels + level_size * cur, j, lim, cw, cv);
-                found = j < lim;
-            }
+        // The search, among the structural bytes of the current level (nothing
+        // happens at any other byte): a ':' whose key matches (:225-251), or
+        // the ',' before the wanted element (:252-259).  A search that fails
+        // ends the line.
+        cend = lv.end(cur);
+        const P lim = cend < n ? cend : n;
+        const uint64_t* bits = levels + level_size * cur;
+        if (to_key) {
+            j = Scan::template find_key<P>(scope, key, bits, colon, j, lim);
         } else {
-            cw = -1;  // opcodes run next and may change the level
+            j = Scan::template find_comma<P>(file, bits, colon, j, lim, want_index - lv.idx(cur));
+            lv.set_idx(cur, static_cast<P>(want_index));
         }
+        if (j >= lim) return kLineDone;
+        ++j;
     }
     return kLineDone;
 }
@@ -506,6 +491,7 @@ constexpr int64_t kRelLimit = (1ll << 31) - 4096;
 // for lines the 32-bit form cannot hold; a separate function, so that its
 // state does not add to the registers of the 32-bit form's caller.  Writes
 // every one of the res_len entries once.
+template <typename Scan = SeqScan>
 #ifdef __CUDACC__
 static __host__ __device__ __noinline__
 #else
@@ -515,10 +501,10 @@ int run_line_wide(const LineView& v, int64_t line_start, int64_t line_end, const
                   int64_t res_len) {
     LocalLevels lv;
     int stored = 0;
-    const int r = run_line_core<int64_t>(v.file, v.n, v.hi, v.hi < v.n ? kLineDeferred : kLineDone, v.string_index,
-                                         v.levels, v.level_size, v.colon, line_start, line_end, ir, res, 0, lv,
-                                         stored);
-    for (int64_t k = 2 * static_cast<int64_t>(stored); k < res_len; k++) res[k] = -1;
+    const int r = run_line_core<int64_t, LocalLevels, Scan>(v.file, v.n, v.hi, v.hi < v.n ? kLineDeferred : kLineDone,
+                                                            v.string_index, v.levels, v.level_size, v.colon,
+                                                            line_start, line_end, ir, res, 0, lv, stored);
+    for (int64_t k = 2 * static_cast<int64_t>(stored); k < res_len; k++) Scan::store(res, k, -1);
     return r;
 }
 
@@ -533,8 +519,8 @@ int run_line_wide(const LineView& v, int64_t line_start, int64_t line_end, const
 // again in 64 bits.  With a skip_bound, a whitespace skip that runs more
 // than skip_bound bytes past the line's end (into the blank lines after it)
 // stops there too and run_line returns kLineLong, with res partly written,
-// for the caller to evaluate the line again (a warp each, query_kernel.cu).
-template <int D = kLevelSlots>
+// for the caller to evaluate the line again (by a warp, query_kernel.cu).
+template <int D = kLevelSlots, typename Scan = SeqScan>
 GPJ_HD int run_line(const LineView& v, int64_t line_start, int64_t line_end, const uint8_t* ir, int64_t* res,
                     int64_t res_len, int64_t rel_limit = kRelLimit, int64_t skip_bound = -1) {
     const int64_t base = line_start & ~static_cast<int64_t>(63);
@@ -548,17 +534,17 @@ GPJ_HD int run_line(const LineView& v, int64_t line_start, int64_t line_end, con
         const int skip_end = clamped || v.hi < v.n ? kLineDeferred : kLineDone;
         const int64_t w = base >> 6;
         RegLevelsT<D, int32_t> lv;
-        const int r = run_line_core<int32_t>(v.file + base, n, hi, skip_end, v.string_index + w, v.levels + w,
-                                             v.level_size, v.colon ? v.colon + w : nullptr,
-                                             static_cast<int32_t>(line_start - base),
-                                             static_cast<int32_t>(line_end - base), ir, res, base, lv, stored);
+        const int r = run_line_core<int32_t, RegLevelsT<D, int32_t>, Scan>(
+            v.file + base, n, hi, skip_end, v.string_index + w, v.levels + w, v.level_size,
+            v.colon ? v.colon + w : nullptr, static_cast<int32_t>(line_start - base),
+            static_cast<int32_t>(line_end - base), ir, res, base, lv, stored);
         if (r != kLineDeferred || !clamped || v.hi < v.n) {
-            for (int64_t k = 2 * static_cast<int64_t>(stored); k < res_len; k++) res[k] = -1;
+            for (int64_t k = 2 * static_cast<int64_t>(stored); k < res_len; k++) Scan::store(res, k, -1);
             return r;
         }
         if (skip_bound >= 0) return kLineLong;
     }
-    return run_line_wide(v, line_start, line_end, ir, res, res_len);
+    return run_line_wide<Scan>(v, line_start, line_end, ir, res, res_len);
 }
 
 // Deepest level a validated query's bytecode reaches (its MOVE_DOWNs).

@@ -18,7 +18,7 @@ struct LongItem {
 };
 
 // Where the thread-per-line kernels put lines longer than `bytes`, which a
-// whole warp then evaluates (find_value_long): `items` holds `cap` entries,
+// whole warp then evaluates (find_value_warp_kernel): `items` holds `cap` entries,
 // `count` (zeroed before the launch) counts them; items past `cap` are
 // evaluated by their thread.  items == nullptr: no line is handed over.
 struct LongLines {
@@ -36,6 +36,12 @@ struct LongLines {
 constexpr int kQueryThreads = 128;
 template <int D>
 constexpr int kQueryMinCtas = D <= 5 ? 7 : (D <= 9 ? 6 : 4);
+// The same for the warp-per-line kernels, and the CTAs per SM they launch
+// for the handed-over lines (whose number the host does not know).
+constexpr int kWarpThreads = 64;
+template <int D>
+constexpr int kWarpMinCtas = D <= 5 ? 12 : (D <= 9 ? 10 : 8);
+constexpr int kListCtasPerSm = 8;
 
 struct QueryParams {
     const uint8_t* file;
@@ -67,12 +73,16 @@ struct QueryParams {
     // deepest level of the launch's queries (sizes the interpreter's
     // register state)
     int depth;
+    // every line by a warp (query_by_warp; not with `range`): one launch of
+    // the warp-per-line kernel alone
+    bool by_warp;
     LongLines long_lines;
 };
 
-// find_value over the launch's lines, then (when p.long_lines.items is set)
-// the long lines a warp each, with `long_grid` CTAs.
-cudaError_t launch_find_value(const QueryParams& p, int grid, int long_grid, cudaStream_t stream);
+// find_value over the launch's lines: a thread per (line, query) with `grid`
+// CTAs, then (when p.long_lines.items is set) the long lines a warp each with
+// `warp_grid` CTAs; or, by_warp, all lines a warp each.
+cudaError_t launch_find_value(const QueryParams& p, int grid, int warp_grid, cudaStream_t stream);
 // Resident CTAs per SM of the find_value kernel for queries of that depth.
 int find_value_max_ctas_per_sm(int depth);
 
@@ -93,18 +103,22 @@ struct QueryFile {
     int slots;
     int64_t* out;
     int64_t out_lines;
-    // first of the file's items in the batch: ceil(num_lines / 32) blocks of
-    // 32 lines x num_queries (a multiple of 32, so no warp spans two files)
+    // first of the file's items in the batch's thread-per-line launch:
+    // ceil(num_lines / 32) blocks of 32 lines x num_queries (a multiple of 32,
+    // so no warp spans two files), none for a file whose lines get a warp each
     int64_t item_begin;
     const uint64_t* colon;  // optional, as QueryParams::colon
+    // first of its (line, query) pairs in the warp-per-line launch (none for
+    // the other files)
+    int64_t warp_begin;
 };
 
 // Every (line, query) item of every file of the batch (`files`: device
-// array, ascending item_begin, total_items items in all; `depth` the deepest
-// level of any of their queries), one per thread:
-// a warp's lanes run one query on 32 lines of one file, and the warps of a
-// block of lines run its queries side by side.
-cudaError_t launch_find_value_batch(const QueryFile* files, int nfiles, int64_t total_items, int depth,
-                                    const LongLines& long_lines, int grid, int long_grid, cudaStream_t stream);
+// array, ascending item_begin and warp_begin; `items` thread and `warp_items`
+// warp items in all; `depth` the deepest level of any of their queries).  A
+// thread-per-line warp's lanes run one query on 32 lines of one file, and the
+// warps of a block of lines run its queries side by side.
+cudaError_t launch_find_value_batch(const QueryFile* files, int nfiles, int64_t items, int64_t warp_items, int depth,
+                                    const LongLines& long_lines, int grid, int warp_grid, cudaStream_t stream);
 
 }  // namespace gpj
