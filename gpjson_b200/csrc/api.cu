@@ -26,6 +26,7 @@
 #include "index_kernel.h"
 #include "jsonpath.h"
 #include "query_kernel.h"
+#include "query_program.h"
 #include "values.h"
 
 namespace {
@@ -110,10 +111,15 @@ struct gpj_file {
     uint8_t* d_owned = nullptr;
     int64_t n = 0;
     int64_t words = 0;
+    // words from one level's bitmap to the next, and allocated for each other
+    // bitmap: find_value reads four aligned words at a time
+    int64_t stride = 0;
 
     uint64_t* d_str = nullptr;
-    uint64_t* d_colon = nullptr;  // ':' outside strings, for find_value's key searches
-    bool colon_valid = false;     // d_colon belongs to the current index
+    // for find_value's key searches (IndexParams::marks, odd)
+    uint64_t* d_marks = nullptr;
+    uint32_t* d_odd = nullptr;
+    bool marks_valid = false;  // they belong to the current index
     uint64_t* d_lvl = nullptr;
     int lvl_cap = 0;
     int64_t* d_nl = nullptr;
@@ -123,8 +129,9 @@ struct gpj_file {
     int num_levels = 0;
     int64_t num_lines = 0;
 
-    // uploaded bytecode (cached across calls with identical queries)
+    // uploaded queries (kept across calls with identical ones)
     std::vector<uint8_t> ir_host;
+    size_t ir_bytecode = 0;  // bytes of it that are offsets and bytecode; then the programs
     int ir_depth = 0;  // deepest level of the uploaded queries
     uint8_t* d_ir = nullptr;
     size_t d_ir_cap = 0;
@@ -430,17 +437,18 @@ int finish_tiles(gpj_ctx* ctx, const gpj::IndexParams& p, const TileScratch& ts)
 // same pass when given), and again with the exact kernel when the input is
 // not well-formed NDJSON.  *lines receives the line count; *queries_done
 // tells whether every line's query results were written.
-// d_colon (optional) receives the ':' bitmap when the standalone kernel
-// builds the index; *colon_valid (optional) tells whether it did.
+// `level_stride`: words from one level's bitmap to the next.
+// d_marks and d_odd (optional) receive the key marks when the standalone
+// kernel builds the index; *marks_valid (optional) tells whether it did.
 // *exact_only (optional, in and out): the input needs the exact kernel (a
 // line kernel flagged it before, so later builds of the same input skip
 // straight to the exact kernel).
 int run_index(gpj_ctx* ctx, const uint8_t* d_file, int64_t n, int num_levels, uint64_t* d_str,
-              uint64_t* d_lvl, int64_t* d_nl, int64_t nl_cap, int64_t* lines, const FusedQueries* fq = nullptr,
-              bool* queries_done = nullptr, uint64_t* d_colon = nullptr, bool* colon_valid = nullptr,
-              bool* exact_only = nullptr) {
+              uint64_t* d_lvl, int64_t level_stride, int64_t* d_nl, int64_t nl_cap, int64_t* lines,
+              const FusedQueries* fq = nullptr, bool* queries_done = nullptr, uint64_t* d_marks = nullptr, uint32_t* d_odd = nullptr,
+              bool* marks_valid = nullptr, bool* exact_only = nullptr) {
     if (queries_done) *queries_done = false;
-    if (colon_valid) *colon_valid = false;
+    if (marks_valid) *marks_valid = false;
     if (n == 0) {
         if (nl_cap > 0) GPJ_CUDA(ctx, cudaMemsetAsync(d_nl, 0, 8, ctx->stream));
         GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -453,7 +461,7 @@ int run_index(gpj_ctx* ctx, const uint8_t* d_file, int64_t n, int num_levels, ui
     p.ntiles = (n + gpj::kIndexTileBytes - 1) / gpj::kIndexTileBytes;
     p.string_index = d_str;
     p.leveled = d_lvl;
-    p.level_size = (n + 63) / 64;
+    p.level_size = level_stride;
     p.num_levels = num_levels;
     p.newlines = d_nl;
     p.newline_cap = nl_cap;
@@ -499,7 +507,8 @@ int run_index(gpj_ctx* ctx, const uint8_t* d_file, int64_t n, int num_levels, ui
             fused.tile_end = fused.ntiles;
             fused.newline_bits = ts.bits;
             fused.tile_newlines = ts.counts;
-            fused.colon = d_colon;
+            fused.marks = d_marks;
+            fused.odd = d_odd;
             fused.status = ctx->d_status;
             rc = set_tile_states(ctx, &fused, fused.ntiles);
             if (!rc) rc = launch_tiles(ctx, fused);
@@ -521,7 +530,7 @@ int run_index(gpj_ctx* ctx, const uint8_t* d_file, int64_t n, int num_levels, ui
     rc = status_error(ctx, errs);
     if (rc) return rc;
     *lines = static_cast<int64_t>(ctx->h_status[0]);
-    if (colon_valid) *colon_valid = d_colon && !exact && !(fq && fq->nq > 0);
+    if (marks_valid) *marks_valid = d_marks && !exact && !(fq && fq->nq > 0);
     if (queries_done && fq && fq->nq > 0)
         *queries_done = !exact && !(errs & (gpj::kErrDeferred | gpj::kErrOutOverflow)) && *lines <= fq->out_lines;
     return GPJ_OK;
@@ -547,16 +556,22 @@ int make_file(gpj_ctx* ctx, int64_t n, gpj_file** out) {
     f->ctx = ctx;
     f->n = n;
     f->words = (n + 63) / 64;
+    f->stride = (f->words + 15) / 16 * 16;
     *out = f;
     return GPJ_OK;
 }
 
-// Packs validated bytecode as [int32 offsets (16-byte padded)][bytes] and
-// uploads it unless the previous upload was identical.
+// Offsets of a call's queries, padded to 16 bytes.
+size_t offsets_bytes(size_t nq) { return (nq * 4 + 15) / 16 * 16; }
+
+// Packs validated bytecode as [int32 offsets (16-byte padded)][bytes] for the
+// queries evaluated by the line kernel, then (ir_bytecode) the queries'
+// programs the same way for find_value, and uploads both unless the previous
+// upload was identical.
 int upload_queries(gpj_ctx* ctx, gpj_file* f, int nq, const uint8_t* const* bc, const size_t* len,
                    int slots, int* depth_needed) {
     std::vector<uint8_t> packed;
-    const size_t header = ((static_cast<size_t>(nq) * 4 + 15) / 16) * 16;
+    const size_t header = offsets_bytes(static_cast<size_t>(nq));
     packed.resize(header);
     int deepest = 0;
     for (int q = 0; q < nq; q++) {
@@ -570,8 +585,16 @@ int upload_queries(gpj_ctx* ctx, gpj_file* f, int nq, const uint8_t* const* bc, 
         std::memcpy(packed.data() + 4 * q, &off, 4);
         packed.insert(packed.end(), bc[q], bc[q] + len[q]);
     }
+    packed.resize((packed.size() + 15) / 16 * 16, 0);
+    const size_t programs = packed.size();
+    packed.resize(programs + header, 0);
+    for (int q = 0; q < nq; q++) {
+        const int32_t off = gpj::append_program(bc[q], &packed) - static_cast<int32_t>(programs + header);
+        std::memcpy(packed.data() + programs + 4 * q, &off, 4);
+    }
     *depth_needed = deepest;
     f->ir_depth = deepest;
+    f->ir_bytecode = programs;
     if (packed == f->ir_host && f->d_ir) return GPJ_OK;
     if (packed.size() > f->d_ir_cap) {
         device_free(ctx, f->d_ir);
@@ -619,7 +642,6 @@ int warp_grid(const gpj_ctx* ctx, int64_t items, bool listed) {
 int launch_query(gpj_ctx* ctx, gpj_file* f, int nq, int slots, int64_t* d_out, int64_t out_lines,
                  const int64_t* d_range = nullptr, bool last = false) {
     cudaStream_t stream = ctx->stream;
-    const size_t header = ((static_cast<size_t>(nq) * 4 + 15) / 16) * 16;
     gpj::QueryParams p{};
     p.file = f->d_data;
     p.n = f->n;
@@ -627,9 +649,9 @@ int launch_query(gpj_ctx* ctx, gpj_file* f, int nq, int slots, int64_t* d_out, i
     p.num_lines = f->num_lines;
     p.string_index = f->d_str;
     p.leveled = f->d_lvl;
-    p.level_size = f->words;
-    p.bytecode = f->d_ir + header;
-    p.offsets = reinterpret_cast<const int32_t*>(f->d_ir);
+    p.level_size = f->stride;
+    p.programs = f->d_ir + f->ir_bytecode + offsets_bytes(static_cast<size_t>(nq));
+    p.offsets = reinterpret_cast<const int32_t*>(f->d_ir + f->ir_bytecode);
     p.num_queries = nq;
     p.slots = slots;
     p.out = d_out;
@@ -637,11 +659,13 @@ int launch_query(gpj_ctx* ctx, gpj_file* f, int nq, int slots, int64_t* d_out, i
     p.range = d_range;
     p.last = last ? 1 : 0;
     p.newline_cap = f->nl_cap;
-    p.colon = f->colon_valid ? f->d_colon : nullptr;
+    p.marks = f->marks_valid ? f->d_marks : nullptr;
+    p.odd = f->marks_valid ? f->d_odd : nullptr;
     p.depth = f->ir_depth;
     // (a chunk's lines are not counted yet)
     p.by_warp = !d_range && ctx->tuning.long_line_bytes >= 0 &&
                 gpj::query_by_warp(f->num_lines, f->n, nq, kFewPairs);
+    p.short_lines = !d_range && f->n / gpj::kShortLineBytes < f->num_lines;
     if (!p.by_warp) p.long_lines = long_lines(ctx);
     if (p.long_lines.items)
         GPJ_CUDA(ctx, cudaMemsetAsync(ctx->d_long_count, 0, sizeof(unsigned long long), stream));
@@ -667,15 +691,17 @@ int ensure_index_buffers(gpj_ctx* ctx, gpj_file* f, int num_levels) {
     int rc;
     if (num_levels < 1 || num_levels > GPJ_MAX_LEVELS)
         return fail(ctx, GPJ_ELIMIT, "Invalid number of levels: " + std::to_string(num_levels));
-    if (!f->d_str && (rc = device_alloc(ctx, &f->d_str, static_cast<size_t>(f->words), "cudaMalloc(string index)")))
+    if (!f->d_str && (rc = device_alloc(ctx, &f->d_str, static_cast<size_t>(f->stride), "cudaMalloc(string index)")))
         return rc;
-    if (!f->d_colon && (rc = device_alloc(ctx, &f->d_colon, static_cast<size_t>(std::max<int64_t>(f->words, 1)),
-                                          "cudaMalloc(colon bitmap)")))
+    if (!f->d_marks && (rc = device_alloc(ctx, &f->d_marks, static_cast<size_t>(f->stride), "cudaMalloc(key marks)")))
+        return rc;
+    if (!f->d_odd &&
+        (rc = device_alloc(ctx, &f->d_odd, static_cast<size_t>((f->words + 31) / 32), "cudaMalloc(odd words)")))
         return rc;
     if (f->lvl_cap < num_levels) {
         device_free(ctx, f->d_lvl);
         f->lvl_cap = 0;
-        rc = device_alloc(ctx, &f->d_lvl, static_cast<size_t>(f->words) * num_levels, "cudaMalloc(leveled bitmaps)");
+        rc = device_alloc(ctx, &f->d_lvl, static_cast<size_t>(f->stride) * num_levels, "cudaMalloc(leveled bitmaps)");
         if (rc) return rc;
         f->lvl_cap = num_levels;
     }
@@ -694,20 +720,20 @@ int index_pass(gpj_ctx* ctx, gpj_file* f, int num_levels, const FusedQueries* fq
     int rc = ensure_index_buffers(ctx, f, num_levels);
     if (rc) return rc;
     f->indexed = false;
-    f->colon_valid = false;
+    f->marks_valid = false;
     const double t0 = now_ms();
     GPJ_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     int64_t lines = 0;
-    rc = run_index(ctx, f->d_data, f->n, num_levels, f->d_str, f->d_lvl, f->d_nl, f->nl_cap, &lines, fq,
-                   queries_done, f->d_colon, &f->colon_valid, &f->exact_only);
+    rc = run_index(ctx, f->d_data, f->n, num_levels, f->d_str, f->d_lvl, f->stride, f->d_nl, f->nl_cap, &lines, fq,
+                   queries_done, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only);
     if (rc) return rc;
     if (lines > f->nl_cap) {  // more lines than the first guess: size exactly and rebuild
         device_free(ctx, f->d_nl);
         f->nl_cap = lines;
         rc = device_alloc(ctx, &f->d_nl, static_cast<size_t>(lines), "cudaMalloc(newline index)");
         if (rc) return rc;
-        rc = run_index(ctx, f->d_data, f->n, num_levels, f->d_str, f->d_lvl, f->d_nl, f->nl_cap, &lines, fq,
-                       queries_done, f->d_colon, &f->colon_valid, &f->exact_only);
+        rc = run_index(ctx, f->d_data, f->n, num_levels, f->d_str, f->d_lvl, f->stride, f->d_nl, f->nl_cap, &lines, fq,
+                       queries_done, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only);
         if (rc) return rc;
     }
     rc = end_phase(ctx, fq && fq->nq ? "index_and_query" : "build_index", t0);
@@ -756,7 +782,7 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
     int rc = ensure_index_buffers(ctx, f, num_levels);
     if (rc) return rc;
     f->indexed = false;
-    f->colon_valid = false;
+    f->marks_valid = false;
     const double t0 = now_ms();
     GPJ_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     const int64_t chunk_bytes = kChunkUnit * chunk_units;
@@ -767,8 +793,8 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         if (n > 0 && !resident)
             GPJ_CUDA(ctx, cudaMemcpyAsync(f->d_owned, host, static_cast<size_t>(n), cudaMemcpyHostToDevice,
                                           ctx->stream));
-        rc = run_index(ctx, f->d_data, n, num_levels, f->d_str, f->d_lvl, f->d_nl, f->nl_cap, &lines, nullptr,
-                           nullptr, f->d_colon, &f->colon_valid, &f->exact_only);
+        rc = run_index(ctx, f->d_data, n, num_levels, f->d_str, f->d_lvl, f->stride, f->d_nl, f->nl_cap, &lines, nullptr,
+                           nullptr, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only);
         if (rc) return rc;
     } else {
         while (!resident && static_cast<int64_t>(ctx->chunk_events.size()) < nchunks) {
@@ -782,14 +808,15 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         p.ntiles = (n + gpj::kStandaloneTileBytes - 1) / gpj::kStandaloneTileBytes;
         p.string_index = f->d_str;
         p.leveled = f->d_lvl;
-        p.level_size = f->words;
+        p.level_size = f->stride;
         p.num_levels = num_levels;
         p.newlines = f->d_nl;
         p.newline_cap = f->nl_cap;
         p.materialize = 1;
         p.avail = n;
-        p.colon = f->d_colon;
-        f->colon_valid = true;  // the chunks' queries read it as their tiles write it
+        p.marks = f->d_marks;
+        p.odd = f->d_odd;
+        f->marks_valid = true;  // the chunks' queries read it as their tiles write it
         TileScratch ts;
         rc = alloc_tile_scratch(ctx, n, &ts);
         if (!rc) rc = set_tile_states(ctx, &p, p.ntiles);
@@ -806,7 +833,7 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         if (rc) {
             free_tile_scratch(ctx, &ts);
             device_free(ctx, d_lines);
-            f->colon_valid = false;
+            f->marks_valid = false;
             return rc;
         }
         p.status = ctx->d_status;
@@ -853,7 +880,7 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         free_tile_scratch(ctx, &ts);
         device_free(ctx, d_lines);
         if (rc) {
-            f->colon_valid = false;
+            f->marks_valid = false;
             if (!resident) cudaStreamSynchronize(ctx->copy_stream);
             return rc;
         }
@@ -861,11 +888,11 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         lines = static_cast<int64_t>(ctx->h_status[0]);
         if (errs & (gpj::kErrIrregular | gpj::kErrLongLine)) {
             // the whole input is on the device now: index it in one launch (exact fallback inside)
-            rc = run_index(ctx, f->d_data, n, num_levels, f->d_str, f->d_lvl, f->d_nl, f->nl_cap, &lines, nullptr,
-                           nullptr, f->d_colon, &f->colon_valid, &f->exact_only);
+            rc = run_index(ctx, f->d_data, n, num_levels, f->d_str, f->d_lvl, f->stride, f->d_nl, f->nl_cap, &lines, nullptr,
+                           nullptr, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only);
             if (rc) return rc;
         } else if ((rc = status_error(ctx, errs))) {
-            f->colon_valid = false;
+            f->marks_valid = false;
             return rc;
         } else if (cq && lines <= f->nl_cap && lines <= cq->out_lines && queries_done) {
             *queries_done = true;
@@ -876,8 +903,8 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         f->nl_cap = lines;
         rc = device_alloc(ctx, &f->d_nl, static_cast<size_t>(lines), "cudaMalloc(newline index)");
         if (rc) return rc;
-        rc = run_index(ctx, f->d_data, n, num_levels, f->d_str, f->d_lvl, f->d_nl, f->nl_cap, &lines, nullptr,
-                           nullptr, f->d_colon, &f->colon_valid, &f->exact_only);
+        rc = run_index(ctx, f->d_data, n, num_levels, f->d_str, f->d_lvl, f->stride, f->d_nl, f->nl_cap, &lines, nullptr,
+                           nullptr, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only);
         if (rc) return rc;
     }
     rc = end_phase(ctx, resident ? "index_and_query" : "load_and_index", t0);
@@ -941,10 +968,10 @@ int index_and_query(gpj_ctx* ctx, gpj_file* f, int num_levels, int nq, const uin
     FusedQueries fq;
     fq.nq = nq;
     fq.slots = slots;
-    const size_t header = ((static_cast<size_t>(nq) * 4 + 15) / 16) * 16;
+    const size_t header = offsets_bytes(static_cast<size_t>(nq));
     fq.offsets = reinterpret_cast<const int32_t*>(f->d_ir);
     fq.bytecode = f->d_ir + header;
-    fq.bytecode_bytes = static_cast<int>(f->ir_host.size() - header);
+    fq.bytecode_bytes = static_cast<int>(f->ir_bytecode - header);
     fq.out = d_out;
     fq.out_lines = out_lines;
     bool done = false;
@@ -1473,7 +1500,8 @@ void gpj_file_release(gpj_file* f) {
         gpj_ctx* ctx = f->ctx;
         device_free(ctx, f->d_owned);
         device_free(ctx, f->d_str);
-        device_free(ctx, f->d_colon);
+        device_free(ctx, f->d_marks);
+        device_free(ctx, f->d_odd);
         device_free(ctx, f->d_lvl);
         device_free(ctx, f->d_nl);
         device_free(ctx, f->d_ir);
@@ -1532,7 +1560,8 @@ int gpj_index_copy_leveled_bitmaps(gpj_ctx* ctx, const gpj_file* f, uint64_t* ho
     const int64_t total = f->words * f->num_levels;
     if (count < total) return fail(ctx, GPJ_EINVAL, "host buffer too small");
     if (total == 0) return GPJ_OK;
-    GPJ_CUDA(ctx, cudaMemcpyAsync(host, f->d_lvl, total * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    GPJ_CUDA(ctx, cudaMemcpy2DAsync(host, f->words * 8, f->d_lvl, f->stride * 8, f->words * 8, f->num_levels,
+                                    cudaMemcpyDeviceToHost, ctx->stream));
     GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return GPJ_OK;
 }
@@ -1552,7 +1581,7 @@ int gpj_build_index_device(gpj_ctx* ctx, const void* d_file, int64_t n, int num_
     const double t0 = now_ms();
     GPJ_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     rc = run_index(ctx, static_cast<const uint8_t*>(d_file), n, num_levels, d_string_index, d_leveled,
-                   d_newlines, newline_cap, num_lines);
+                   (n + 63) / 64, d_newlines, newline_cap, num_lines);
     if (rc) return rc;
     rc = end_phase(ctx, "build_index", t0);
     if (rc) return rc;
@@ -1842,7 +1871,7 @@ int batch_index(gpj_ctx* ctx, std::vector<gpj_batch::FileRun>& files) {
         if (f->ctx != ctx) GPJ_CUDA(ctx, cudaStreamSynchronize(f->ctx->stream));
         if ((rc = ensure_index_buffers(ctx, f, levels))) return rc;
         f->indexed = false;
-        f->colon_valid = false;
+        f->marks_valid = false;
         if (f->n == 0) continue;  // indexed alone below
         batched.push_back(f);
         total_tiles += (f->n + gpj::kStandaloneTileBytes - 1) / gpj::kStandaloneTileBytes;
@@ -1871,8 +1900,8 @@ int batch_index(gpj_ctx* ctx, std::vector<gpj_batch::FileRun>& files) {
             for (int i = 0; i < nb; i++) {
                 gpj_file* f = batched[i];
                 const int64_t ntiles = (f->n + gpj::kStandaloneTileBytes - 1) / gpj::kStandaloneTileBytes;
-                tf.push_back(gpj::TileFile{f->d_data, f->n, f->n, f->d_str, f->d_lvl, f->words, bits + word,
-                                           status + 2 * i, tile, f->d_colon});
+                tf.push_back(gpj::TileFile{f->d_data, f->n, f->n, f->d_str, f->d_lvl, f->stride, bits + word,
+                                           status + 2 * i, tile, nullptr, f->d_marks, f->d_odd});
                 lf.push_back(gpj::LineFile{bits + word, f->words, f->d_nl, f->nl_cap, status + 2 * i, tile, ntiles});
                 tile += ntiles;
                 word += f->words;
@@ -1934,7 +1963,7 @@ int batch_index(gpj_ctx* ctx, std::vector<gpj_batch::FileRun>& files) {
             f->num_lines = lines;
             f->num_levels = levels;
             f->indexed = true;
-            f->colon_valid = true;
+            f->marks_valid = true;
         }
     }
     for (gpj_file* f : need)
@@ -2016,7 +2045,7 @@ int gpj_batch_run(gpj_batch* b) {
     // one find_value launch over every line of every file
     const double t0 = now_ms();
     GPJ_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-    std::vector<uint8_t> blob;  // per file: [int32 offsets (16-byte padded)][bytecode]
+    std::vector<uint8_t> blob;  // per file: [int32 offsets (16-byte padded)][programs]
     std::vector<size_t> blob_at(b->files.size());
     size_t total_out = 0;
     int64_t total_items = 0, warp_items = 0, pairs = 0;
@@ -2024,14 +2053,11 @@ int gpj_batch_run(gpj_batch* b) {
         auto& fr = b->files[i];
         const size_t nq = fr.queries.size();
         blob_at[i] = blob.size();
-        const size_t header = ((nq * 4 + 15) / 16) * 16;
-        blob.resize(blob.size() + header, 0);
-        size_t code = 0;
+        const size_t begin = blob.size() + offsets_bytes(nq);
+        blob.resize(begin, 0);
         for (size_t q = 0; q < nq; q++) {
-            const int32_t off = static_cast<int32_t>(code);
+            const int32_t off = gpj::append_program(fr.queries[q]->bytecode.data(), &blob) - static_cast<int32_t>(begin);
             std::memcpy(blob.data() + blob_at[i] + 4 * q, &off, 4);
-            blob.insert(blob.end(), fr.queries[q]->bytecode.begin(), fr.queries[q]->bytecode.end());
-            code += fr.queries[q]->bytecode.size();
         }
         blob.resize((blob.size() + 15) / 16 * 16, 0);
         fr.lines = fr.file->num_lines;
@@ -2065,7 +2091,7 @@ int gpj_batch_run(gpj_batch* b) {
                            static_cast<uint64_t>(reinterpret_cast<uintptr_t>(f->d_nl)),
                            static_cast<uint64_t>(reinterpret_cast<uintptr_t>(f->d_str)),
                            static_cast<uint64_t>(reinterpret_cast<uintptr_t>(f->d_lvl)),
-                           static_cast<uint64_t>(reinterpret_cast<uintptr_t>(f->colon_valid ? f->d_colon : nullptr)),
+                           static_cast<uint64_t>(reinterpret_cast<uintptr_t>(f->marks_valid ? f->d_marks : nullptr)),
                            static_cast<uint64_t>(f->num_lines), static_cast<uint64_t>(f->n)})
             sig.push_back(v);
     }
@@ -2101,12 +2127,13 @@ int gpj_batch_run(gpj_batch* b) {
             auto& fr = b->files[i];
             gpj_file* f = fr.file;
             const size_t nq = fr.queries.size();
-            const size_t header = ((nq * 4 + 15) / 16) * 16;
-            qf.push_back(gpj::QueryFile{f->d_data, f->n, f->d_nl, fr.lines, f->d_str, f->d_lvl, f->words,
+            const size_t header = offsets_bytes(nq);
+            qf.push_back(gpj::QueryFile{f->d_data, f->n, f->d_nl, fr.lines, f->d_str, f->d_lvl, f->stride,
                                         d_blob + blob_at[i] + header,
                                         reinterpret_cast<const int32_t*>(d_blob + blob_at[i]),
                                         static_cast<int>(nq), fr.slots, d_out + fr.out_offset, fr.lines, item,
-                                        f->colon_valid ? f->d_colon : nullptr, warp_item});
+                                        f->marks_valid ? f->d_marks : nullptr,
+                                        f->marks_valid ? f->d_odd : nullptr, warp_item});
             if (fr.by_warp)
                 warp_item += fr.lines * static_cast<int64_t>(nq);
             else

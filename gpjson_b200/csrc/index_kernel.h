@@ -26,12 +26,15 @@ struct TileFile {
     int64_t n;
     int64_t avail;            // bytes [0, avail) readable
     uint64_t* string_index;
-    uint64_t* leveled;        // num_levels * level_size words
+    uint64_t* leveled;        // num_levels bitmaps, level_size words apart
     int64_t level_size;
     uint64_t* newline_bits;
     unsigned long long* status;  // [0] line count, [1] error bits
     int64_t tile_begin;
-    uint64_t* colon;          // optional: ':' outside strings (level_size words)
+    uint64_t* colon;          // line-parallel kernel, optional: ':' outside strings
+    // standalone kernel, optional (both or none): see IndexParams
+    uint64_t* marks;
+    uint32_t* odd;
 };
 
 struct IndexParams {
@@ -39,8 +42,8 @@ struct IndexParams {
     int64_t n;
     int64_t ntiles;
     uint64_t* string_index;  // ceil(n/64)
-    uint64_t* leveled;       // num_levels * level_size
-    int64_t level_size;      // ceil(n/64)
+    uint64_t* leveled;       // num_levels bitmaps, level_size words apart
+    int64_t level_size;      // at least ceil(n/64)
     int num_levels;
     int64_t* newlines;  // newline_cap entries
     int64_t newline_cap;
@@ -62,10 +65,15 @@ struct IndexParams {
     // the newline count of every tile, in place of the newline index.
     uint64_t* newline_bits;
     int32_t* tile_newlines;
-    // Standalone kernel, optional: the ':' bytes outside strings
-    // (ceil(n/64) words), which lets find_value's key searches skip the ','
-    // candidates.
+    // Optional: the ':' bytes outside strings (ceil(n/64) words).
     uint64_t* colon;
+    // Standalone kernel, optional, what find_value's key searches jump by:
+    // `marks` (ceil(n/64) words): the ':' outside strings and the quotes that
+    // open a string; `odd`, one bit per word of 64 bytes (32 words to an
+    // entry): whether the word has a backslash or a ':' outside strings that
+    // is not right after a closing quote (also set where that is not known).
+    uint64_t* marks;
+    uint32_t* odd;
     // Standalone kernel over a batch of files (batch_files > 0): tiles
     // [tile_begin, tile_end) of the whole batch, file table `batch`
     // (ascending tile_begin); status then reports errors that concern no

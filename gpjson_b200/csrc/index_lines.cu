@@ -215,8 +215,9 @@ struct FShared {
     uint8_t bytes[kByteSlots][kSlotBytes];
     TileFile desc[kRing];  // the file of the tile (by tile number modulo kRing)
     uint64_t str[kMaskSlots][kSlotWords];
-    uint64_t colon[kMaskSlots][kSlotWords];
-    uint64_t lv[kMaskSlots][LV][kSlotWords];
+    // (read four words at a time by the interpreter)
+    alignas(32) uint64_t colon[kMaskSlots][kSlotWords];
+    alignas(32) uint64_t lv[kMaskSlots][LV][kSlotWords];
     uint64_t nlmask[kMaskSlots][kTileWords];
     int32_t nlexcl[kMaskSlots][kTileWords];
     int32_t nlpos[kMaskSlots][kMaxTileLines];

@@ -238,6 +238,7 @@ __global__ void __launch_bounds__(kThreads, LV <= 4 ? 5 : (LV <= 8 ? 4 : 3)) til
         // 16-byte halves of each 32 bytes in the other order (4 of 8 bank
         // groups per quarter-warp instead of 2)
         uint64_t open, close, structural, colon, newline, p0;
+        unsigned ballot_b;  // the warp's words with backslashes
         {
             const bool swapped = (lane & 2) != 0;
             const uint4* even = reinterpret_cast<const uint4*>(bytes + 64 * tid + (swapped ? 16 : 0));
@@ -266,7 +267,7 @@ __global__ void __launch_bounds__(kThreads, LV <= 4 ? 5 : (LV <= 8 ? 4 : 3)) til
             // escapes: a word's first byte from the run that ends the word
             // before it; a warp without backslashes can only have its first
             // byte escaped
-            const unsigned ballot_b = __ballot_sync(~0u, bs != 0);
+            ballot_b = __ballot_sync(~0u, bs != 0);
             uint32_t cin = 0;
             if (lane == 0 && (tid > 0 || tile_start > 0) && bytes[64 * tid - 1] == '\\')
                 cin = escape_before(bytes, 64 * tid, F.file, tile_start);
@@ -344,6 +345,16 @@ __global__ void __launch_bounds__(kThreads, LV <= 4 ? 5 : (LV <= 8 ? 4 : 3)) til
         close &= ~in_string;
         structural &= ~in_string;
         colon &= ~in_string;
+        // for find_value's key searches: the marks are the ':' and the quotes
+        // that open a string; a word is odd that has a backslash or a ':'
+        // not right after a closing quote (or not known to be: the first
+        // byte of a warp's words)
+        const uint64_t state_before = (in_string << 1) | static_cast<uint64_t>(s0 ^ s_warp);
+        const uint64_t closing = ~in_string & state_before;
+        const unsigned last_closes = __ballot_sync(~0u, static_cast<int>(closing >> 63) != 0);
+        const uint64_t after_closing = (closing << 1) | ((lane ? last_closes >> (lane - 1) : 0u) & 1u);
+        const unsigned odd = ballot_b | __ballot_sync(~0u, (colon & ~after_closing) != 0);
+        const uint64_t marks = colon | (in_string & ~state_before);
         const uint32_t open_lo = static_cast<uint32_t>(open), open_hi = static_cast<uint32_t>(open >> 32);
         const uint32_t close_lo = static_cast<uint32_t>(close), close_hi = static_cast<uint32_t>(close >> 32);
         const int o_lo = popc32(open_lo), c_lo = popc32(close_lo);
@@ -411,7 +422,10 @@ __global__ void __launch_bounds__(kThreads, LV <= 4 ? 5 : (LV <= 8 ? 4 : 3)) til
             const uint64_t valid = tail ? bits_between(0, F.n - tile_start - 64 * tid) : ~0ull;
             F.string_index[word] = in_string & valid;
             F.newline_bits[word] = newline;
-            if (F.colon) F.colon[word] = colon;
+            if (F.marks) {
+                F.marks[word] = marks;
+                if (lane == 0) F.odd[word >> 5] = odd;
+            }
 #pragma unroll
             for (int l = 0; l < LV; l++)
                 if (l < p.num_levels) F.leveled[F.level_size * l + word] = lv[l];

@@ -155,7 +155,7 @@ cudaError_t launch_newline_index_range(const IndexParams& p, int64_t* offsets, i
                                                                                        blk0);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const LineFile one{p.newline_bits, p.level_size, p.newlines, p.newline_cap, p.status, 0, ntiles};
+    const LineFile one{p.newline_bits, (p.n + 63) / 64, p.newlines, p.newline_cap, p.status, 0, ntiles};
     newline_scatter_kernel<<<grid, 256, 0, stream>>>(p.tile_newlines, offsets, p.tile_state, ntiles, t0, t1, one,
                                                      nullptr, 0, lines_done);
     return cudaGetLastError();

@@ -28,6 +28,15 @@ constexpr int64_t kWarpLineBytes = 4096;
 GPJ_HD bool query_item(int64_t k, int64_t item_begin, int64_t num_lines, int num_queries, int64_t stride,
                        int64_t* line, int* query) {
     const int64_t group = 32 * static_cast<int64_t>(num_queries);
+    if (item_begin + k < INT32_MAX && stride < INT32_MAX) {
+        // (three divisions an item, several times cheaper in 32 bits)
+        const uint32_t g = static_cast<uint32_t>(group), b = static_cast<uint32_t>(k) / g;
+        const uint32_t r = static_cast<uint32_t>(k) - b * g;
+        const uint32_t round = (static_cast<uint32_t>(item_begin) + b * g) / static_cast<uint32_t>(stride);
+        *query = static_cast<int>(((r >> 5) + round) % static_cast<uint32_t>(num_queries));
+        *line = (static_cast<int64_t>(b) << 5) + (r & 31);
+        return *line < num_lines;
+    }
     const int64_t b = k / group;
     const int64_t r = k - b * group;
     *query = static_cast<int>(((r >> 5) + (item_begin + b * group) / stride) % num_queries);
@@ -47,5 +56,9 @@ GPJ_HD int64_t query_items(int64_t num_lines, int num_queries) {
 GPJ_HD bool query_by_warp(int64_t lines, int64_t bytes, int num_queries, int64_t few) {
     return lines * num_queries <= few || bytes / kWarpLineBytes >= lines;
 }
+
+// Mean line length under which a thread reads one bitmap word at a time
+// (Words, interp.cuh: a line of under four words rarely wants the next).
+constexpr int64_t kShortLineBytes = 256;
 
 }  // namespace gpj

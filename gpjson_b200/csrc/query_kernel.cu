@@ -15,6 +15,14 @@
 //
 // Long lines, and all lines where there are few (query_by_warp), get a warp
 // each in a second kernel: its searches look at 2 KiB of bitmap per step.
+//
+// Bound by the waits for cache misses (long scoreboard 7 of 13 stall cycles
+// per instruction; DRAM 2.3 TB/s, ALU 50 %).  256 MiB of tweets, 4 queries:
+// 145 us and 70 M warp instructions; 271 us and 127 M when every key
+// candidate was checked byte by byte, 197 us and 76 M when each cost a load
+// of the file's bytes before it, before candidates were judged by their
+// keys' lengths (KeyScope) and the queries decoded on the host
+// (query_program.h).
 #include <cstdint>
 
 #include "interp.cuh"
@@ -93,14 +101,14 @@ struct WarpScan {
         });
     }
     // each lane checks the candidates of its own word
-    template <typename P>
-    __device__ static P find_key(const KeyScope<P>& v, const Key& key, const uint64_t* bits, const uint64_t* colon,
+    template <typename P, bool kWords>
+    __device__ static P find_key(const KeyScope<P>& v, const Key<kWords>& key, const uint64_t* bits, const uint64_t* colon,
                                  P from, P limit) {
         return walk<P>(bits, colon, 0, from, limit, [&](P w, uint64_t x) -> P {
             P found = -1;
             for (; x && found < 0; x &= x - 1) {
                 const P p = ((w + (threadIdx.x & 31)) << 6) + ctz64(x);
-                if (key_may_be_at<P>(v, key, p) && (colon || v.file[p] == ':') && key_at<P>(v, key, p)) found = p;
+                if ((colon || v.file[p] == ':') && key_at<P>(v, key, p)) found = p;
             }
             const unsigned hit = __ballot_sync(~0u, found >= 0);
             return hit ? __shfl_sync(~0u, found, __ffs(static_cast<int>(hit)) - 1) : -1;
@@ -190,11 +198,11 @@ __device__ __forceinline__ int64_t handed_over(const LongLines& L) {
 }
 
 // D: level slots of the interpreter's register state (level_slots_for_depth
-// of the deepest query of the launch).
-template <int D>
+// of the deepest query of the launch); K: bitmap words read at a time.
+template <int D, int K>
 __global__ void __launch_bounds__(kQueryThreads, kQueryMinCtas<D>) find_value_kernel(QueryParams p) {
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    const LineView view{p.file, p.n, p.string_index, p.leveled, p.level_size, p.n, p.colon};
+    const LineView view{p.file, p.n, p.string_index, p.leveled, p.level_size, p.n, p.marks, p.odd};
     const int64_t per_line = 2 * static_cast<int64_t>(p.slots);
     // lines [first, first + lines); the file's last line ends at p.n
     int64_t first = 0, lines = p.num_lines, file_lines = p.num_lines;
@@ -215,11 +223,11 @@ __global__ void __launch_bounds__(kQueryThreads, kQueryMinCtas<D>) find_value_ke
         const int64_t end = to_eof ? p.n : p.newlines[i + 1];
         if (p.long_lines.items && end - start > p.long_lines.bytes && hand_over(p.long_lines, i, 0, q)) continue;
         int64_t* res = p.out + (static_cast<int64_t>(q) * p.out_lines + i) * per_line;
-        const uint8_t* ir = p.bytecode + p.offsets[q];
+        const ProgramCode ir{p.programs + p.offsets[q]};
         // writes every slot once, unless a whitespace skip runs far past the
         // line (then a warp evaluates it again)
-        if (run_line<D>(view, start, end, ir, res, per_line, kRelLimit,
-                        p.long_lines.items ? p.long_lines.bytes : -1) == kLineLong &&
+        if (run_line<D, SeqScanOf<K>>(view, start, end, ir, res, per_line, kRelLimit,
+                                      p.long_lines.items ? p.long_lines.bytes : -1) == kLineLong &&
             !hand_over(p.long_lines, i, 0, q))
             run_line_wide(view, start, end, ir, res, per_line);
     }
@@ -232,7 +240,7 @@ __global__ void __launch_bounds__(kWarpThreads, kWarpMinCtas<D>) find_value_warp
     const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     const int64_t own = p.by_warp ? p.num_lines * p.num_queries : 0;
     const int64_t count = own + handed_over(p.long_lines);
-    const LineView view{p.file, p.n, p.string_index, p.leveled, p.level_size, p.n, p.colon};
+    const LineView view{p.file, p.n, p.string_index, p.leveled, p.level_size, p.n, p.marks, p.odd};
     const int64_t per_line = 2 * static_cast<int64_t>(p.slots);
     const int64_t file_lines = p.range ? (p.last ? p.range[1] : INT64_MAX) : p.num_lines;
     for (int64_t k = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; k < count; k += warps) {
@@ -244,7 +252,8 @@ __global__ void __launch_bounds__(kWarpThreads, kWarpMinCtas<D>) find_value_warp
         const int64_t start = p.newlines[it.line];
         const int64_t end = it.line + 1 >= file_lines ? p.n : p.newlines[it.line + 1];
         int64_t* res = p.out + (static_cast<int64_t>(it.query) * p.out_lines + it.line) * per_line;
-        run_line<D, WarpScan>(view, start, end, p.bytecode + p.offsets[it.query], res, per_line);
+        run_line<D, WarpScan>(view, start, end, ProgramCode{p.programs + p.offsets[it.query]}, res,
+                                    per_line);
     }
 }
 
@@ -265,13 +274,13 @@ __global__ void __launch_bounds__(kQueryThreads, kQueryMinCtas<D>) find_value_ba
         int64_t i;
         int q;
         if (!query_item(g - F.item_begin, F.item_begin, F.num_lines, F.num_queries, stride, &i, &q)) continue;
-        const LineView view{F.file, F.n, F.string_index, F.leveled, F.level_size, F.n, F.colon};
+        const LineView view{F.file, F.n, F.string_index, F.leveled, F.level_size, F.n, F.marks, F.odd};
         const int64_t start = F.newlines[i];
         const int64_t end = i + 1 < F.num_lines ? F.newlines[i + 1] : F.n;
         if (long_lines.items && end - start > long_lines.bytes && hand_over(long_lines, i, lo, q)) continue;
         const int64_t per_line = 2 * static_cast<int64_t>(F.slots);
         int64_t* res = F.out + (q * F.out_lines + i) * per_line;
-        const uint8_t* ir = F.bytecode + F.offsets[q];
+        const ProgramCode ir{F.programs + F.offsets[q]};
         if (run_line<D>(view, start, end, ir, res, per_line, kRelLimit, long_lines.items ? long_lines.bytes : -1) ==
                 kLineLong &&
             !hand_over(long_lines, i, lo, q))
@@ -301,12 +310,13 @@ __global__ void __launch_bounds__(kWarpThreads, kWarpMinCtas<D>) find_value_batc
             it = long_lines.items[k - own];
         }
         const QueryFile& F = files[it.file];
-        const LineView view{F.file, F.n, F.string_index, F.leveled, F.level_size, F.n, F.colon};
+        const LineView view{F.file, F.n, F.string_index, F.leveled, F.level_size, F.n, F.marks, F.odd};
         const int64_t start = F.newlines[it.line];
         const int64_t end = it.line + 1 < F.num_lines ? F.newlines[it.line + 1] : F.n;
         const int64_t per_line = 2 * static_cast<int64_t>(F.slots);
         int64_t* res = F.out + (it.query * F.out_lines + it.line) * per_line;
-        run_line<D, WarpScan>(view, start, end, F.bytecode + F.offsets[it.query], res, per_line);
+        run_line<D, WarpScan>(view, start, end, ProgramCode{F.programs + F.offsets[it.query]}, res,
+                                    per_line);
     }
 }
 
@@ -329,7 +339,10 @@ template <int D>
 cudaError_t launch_d(const QueryParams& p, int grid, int warp_grid, cudaStream_t stream) {
     cudaError_t e = cudaSuccess;
     if (!p.by_warp) {
-        find_value_kernel<D><<<grid, kQueryThreads, 0, stream>>>(p);
+        if (p.short_lines)
+            find_value_kernel<D, 1><<<grid, kQueryThreads, 0, stream>>>(p);
+        else
+            find_value_kernel<D, 2><<<grid, kQueryThreads, 0, stream>>>(p);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && (p.by_warp || p.long_lines.items)) {
@@ -369,13 +382,13 @@ int find_value_max_ctas_per_sm(int depth) {
     cudaError_t e;
     switch (level_slots_for_depth(depth)) {
         case 5:
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, find_value_kernel<5>, kQueryThreads, 0);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, find_value_kernel<5, 2>, kQueryThreads, 0);
             break;
         case 9:
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, find_value_kernel<9>, kQueryThreads, 0);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, find_value_kernel<9, 2>, kQueryThreads, 0);
             break;
         default:
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, find_value_kernel<kLevelSlots>, kQueryThreads, 0);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, find_value_kernel<kLevelSlots, 2>, kQueryThreads, 0);
     }
     return e == cudaSuccess ? blocks : -1;
 }

@@ -31,11 +31,13 @@ struct LongLines {
 // Threads per CTA of find_value_kernel and find_value_batch_kernel (a
 // multiple of 32; grids are sized in these CTAs), and the CTAs per SM their
 // register budget is set for, by register-state size D: 7 (at most 72
-// registers) for D = 5, 6 for D = 9, 4 for D = 17.  128-thread CTAs at 72
-// registers keep 28 warps per SM resident where 256-thread CTAs at 80 kept 24.
+// registers) for D = 5, 5 for D = 9 (32 paths over 64 MiB: 309 us, 340 with
+// 6), 4 for D = 17.  Threads wait for their lines' cache misses, more of them
+// spill: 8 CTAs for D = 5 took 1001 us at 2 GiB of tweets where 7 take 1031,
+// but 153 and 78 us at 256 and 64 MiB where they take 155 and 76.
 constexpr int kQueryThreads = 128;
 template <int D>
-constexpr int kQueryMinCtas = D <= 5 ? 7 : (D <= 9 ? 6 : 4);
+constexpr int kQueryMinCtas = D <= 5 ? 7 : (D <= 9 ? 5 : 4);
 // The same for the warp-per-line kernels, and the CTAs per SM they launch
 // for the handed-over lines (whose number the host does not know).
 constexpr int kWarpThreads = 64;
@@ -50,9 +52,9 @@ struct QueryParams {
     int64_t num_lines;
     const uint64_t* string_index;
     const uint64_t* leveled;
-    int64_t level_size;
-    const uint8_t* bytecode;  // all queries back to back
-    const int32_t* offsets;   // start of query q in `bytecode`
+    int64_t level_size;       // words between levels, a multiple of 4 (LineView)
+    const uint8_t* programs;  // all queries' programs (query_program.h)
+    const int32_t* offsets;   // start of query q's there, a multiple of 16
     int num_queries;
     int slots;     // result slots per line (max num_results)
     int64_t* out;       // [num_queries][out_lines][slots][2]
@@ -66,16 +68,19 @@ struct QueryParams {
     const int64_t* range;
     int last;
     int64_t newline_cap;
-    // Optional ':' outside strings (level_size words): key searches jump
-    // between structural colons, index searches between the other
-    // structural bytes (the bytes each search ignores).
-    const uint64_t* colon;
+    // Optional (both or none), IndexParams::marks and odd: key searches jump
+    // between the ':' of keys of the right length, index searches between the
+    // other structural bytes.
+    const uint64_t* marks;
+    const uint32_t* odd;
     // deepest level of the launch's queries (sizes the interpreter's
     // register state)
     int depth;
     // every line by a warp (query_by_warp; not with `range`): one launch of
     // the warp-per-line kernel alone
     bool by_warp;
+    // a thread reads one bitmap word at a time instead of two
+    bool short_lines;
     LongLines long_lines;
 };
 
@@ -97,7 +102,7 @@ struct QueryFile {
     const uint64_t* string_index;
     const uint64_t* leveled;
     int64_t level_size;
-    const uint8_t* bytecode;
+    const uint8_t* programs;
     const int32_t* offsets;
     int num_queries;
     int slots;
@@ -107,7 +112,8 @@ struct QueryFile {
     // ceil(num_lines / 32) blocks of 32 lines x num_queries (a multiple of 32,
     // so no warp spans two files), none for a file whose lines get a warp each
     int64_t item_begin;
-    const uint64_t* colon;  // optional, as QueryParams::colon
+    const uint64_t* marks;  // optional, as in QueryParams
+    const uint32_t* odd;
     // first of its (line, query) pairs in the warp-per-line launch (none for
     // the other files)
     int64_t warp_begin;

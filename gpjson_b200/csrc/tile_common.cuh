@@ -180,7 +180,7 @@ __device__ __forceinline__ void load_slot(const uint8_t* file, int64_t start, in
 __device__ __forceinline__ void fetch_tile_file(const IndexParams& p, int64_t t, TileFile* out) {
     if (p.batch_files == 0) {
         *out = TileFile{p.file,     p.n,     p.avail,        p.string_index, p.leveled,
-                        p.level_size, p.newline_bits, p.status, 0, p.colon};
+                        p.level_size, p.newline_bits, p.status, 0, p.colon, p.marks, p.odd};
         return;
     }
     int lo = 0, hi = p.batch_files - 1;  // last file with tile_begin <= t

@@ -12,6 +12,7 @@
 #include "../../gpjson_b200/csrc/host_io.h"
 #include "../../gpjson_b200/csrc/interp.cuh"
 #include "../../gpjson_b200/csrc/query_items.cuh"
+#include "../../gpjson_b200/csrc/query_program.h"
 #include "../../gpjson_b200/csrc/word_ops.cuh"
 
 using namespace gpj;
@@ -227,6 +228,30 @@ void hs_find_values(const uint8_t* f, int64_t n, const int64_t* nl, int64_t line
                 run_line<kLevelSlots>(v, start, end, irs[q], res, slots * 2, packed == 2 ? 64 : kRelLimit);
             }
         }
+    }
+}
+
+// The query's program on the standalone index kernel's key marks and odd
+// words (LineView::odd), as the find_value kernels run it: in 32-bit
+// positions, in 64-bit (how = 1), reading one word at a time (how = 2).
+void hs_find_values_marks(const uint8_t* f, int64_t n, const int64_t* nl, int64_t lines, const uint64_t* str,
+                          const uint64_t* lvl, const uint8_t* ir, int slots, int64_t* out, const uint64_t* marks,
+                          const uint32_t* odd, int how) {
+    const LineView v{f, n, str, lvl, (n + 63) / 64, n, marks, odd};
+    std::vector<uint8_t> blob(5);
+    const int32_t at = append_program(ir, &blob);
+    std::vector<uint64_t> aligned((blob.size() - at + 15) / 8);
+    std::memcpy(aligned.data(), blob.data() + at, blob.size() - at);
+    const ProgramCode code{reinterpret_cast<const uint8_t*>(aligned.data())};
+    for (int64_t i = 0; i < lines; i++) {
+        const int64_t end = i + 1 < lines ? nl[i + 1] : n;
+        int64_t* res = out + i * slots * 2;
+        if (how == 1)
+            run_line_wide(v, nl[i], end, code, res, slots * 2);
+        else if (how == 2)
+            run_line<kLevelSlots, SeqScanOf<1>>(v, nl[i], end, code, res, slots * 2);
+        else
+            run_line_depth(bytecode_depth(ir), v, nl[i], end, code, res, slots * 2);
     }
 }
 
