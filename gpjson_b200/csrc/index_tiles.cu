@@ -36,9 +36,9 @@
 // DRAM at a third of its rate.  The kernel this one replaced (30 KiB tiles
 // with a 2 KiB look-ahead each, word state kept in shared memory between two
 // passes, the level split dealt over the warp by cuts) took 193 us there.
-// Index builds: 2 GiB of tweets 1558 -> 1078 us; 1 GiB with lines up to 1 MiB,
-// which went to the exact kernel before, 1287 -> 975 us; 256 MiB of it at 16
-// levels 900 -> 303 us; 256 MiB of 117-byte lines 269 -> 176 us.
+// Index builds: 2 GiB of tweets 1558 -> 1102 us; 1 GiB with lines up to 1 MiB,
+// which went to the exact kernel before, 1287 -> 888 us; 256 MiB of it at 16
+// levels 900 -> 276 us; 256 MiB of 117-byte lines 269 -> 178 us.
 #include <cstdint>
 
 #include "device_common.cuh"
@@ -211,9 +211,13 @@ __device__ void look_back(const unsigned long long* states, int64_t t, int64_t t
     *d_out = d;
 }
 
-// Registers set the CTAs per SM (one 16 KiB slot each).
+// Registers set the CTAs per SM (one 16 KiB slot each): 40 a thread for up to
+// eight levels, 48 with 16, at the price of a few spilled bytes (5, 4 and 3
+// CTAs, none spilled: 2 GiB of tweets 1114 us instead of 1102, 1 GiB with
+// lines up to 1 MiB at 5 levels 980 instead of 888, 256 MiB of it at 16 levels
+// 302 instead of 276).
 template <int LV>
-__global__ void __launch_bounds__(kThreads, LV <= 4 ? 5 : (LV <= 8 ? 4 : 3)) tile_index_kernel(IndexParams p) {
+__global__ void __launch_bounds__(kThreads, LV <= 8 ? 6 : 5) tile_index_kernel(IndexParams p) {
     __shared__ Shared sh;
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(~0u, tid >> 5, 0);
