@@ -55,6 +55,12 @@ static constexpr int64_t kLongLineBytes = 8192;
 static constexpr int64_t kFewPairs = 1 << 13;
 static constexpr int64_t kFewBatchPairs = 4096;
 
+// gpj_ctx::d_status and what follows it.
+static constexpr size_t kControlBytes = 32;
+
+// Results up to this size reach the host through page-locked memory.
+static constexpr size_t kSmallResult = 1 << 20;
+
 static gpj_tuning default_tuning() {
     gpj_tuning t{};
     t.long_line_bytes = 65536;
@@ -80,8 +86,10 @@ struct gpj_ctx {
     // scratch of the index kernel
     unsigned long long* d_tile_state = nullptr;
     int64_t tile_state_words = 0;
-    unsigned int* d_counter = nullptr;
+    // one block, zeroed with one memset before a build: status words, tile
+    // counters (exact and standalone kernel), the count of handed-over lines
     unsigned long long* d_status = nullptr;
+    unsigned int* d_counter = nullptr;
     unsigned long long* h_status = nullptr;  // pinned, 2 words
     uint32_t epoch = 0;
     int index_occupancy[3] = {0, 0, 0};  // exact kernel, levels <=4, <=8, <=16
@@ -101,6 +109,11 @@ struct gpj_ctx {
     size_t stage_bytes = 0;
 
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // a find_value phase whose end nobody has waited for yet (defer_phase)
+    cudaEvent_t evq0 = nullptr, evq1 = nullptr;
+    bool deferred = false;
+    double deferred_host_ms = 0;
+    uint8_t* h_small = nullptr;  // pinned, kSmallResult bytes
     int64_t launches = 0;
     std::vector<Phase> phases;
 };
@@ -116,7 +129,7 @@ struct gpj_file {
     int64_t stride = 0;
 
     uint64_t* d_str = nullptr;
-    // for find_value's key searches (IndexParams::marks, odd)
+    // for find_value's key searches (IndexParams::marks, odd), after d_str in its allocation
     uint64_t* d_marks = nullptr;
     uint32_t* d_odd = nullptr;
     bool marks_valid = false;  // they belong to the current index
@@ -124,6 +137,8 @@ struct gpj_file {
     int lvl_cap = 0;
     int64_t* d_nl = nullptr;
     int64_t nl_cap = 0;
+    // they lie in d_str's allocation (until more levels or lines are needed)
+    bool lvl_inside = false, nl_inside = false;
     bool indexed = false;
     bool exact_only = false;  // the line kernels flagged this input: index it with the exact kernel
     int num_levels = 0;
@@ -282,20 +297,62 @@ void device_free(gpj_ctx* ctx, T*& p) {
     p = nullptr;
 }
 
+void free_levels(gpj_ctx* ctx, gpj_file* f) {
+    if (!f->lvl_inside) device_free(ctx, f->d_lvl);
+    f->d_lvl = nullptr;
+    f->lvl_cap = 0;
+    f->lvl_inside = false;
+}
+
+void free_newlines(gpj_ctx* ctx, gpj_file* f) {
+    if (!f->nl_inside) device_free(ctx, f->d_nl);
+    f->d_nl = nullptr;
+    f->nl_cap = 0;
+    f->nl_inside = false;
+}
+
+// A newline index of `lines` entries in place of the file's (empty).
+int resize_newlines(gpj_ctx* ctx, gpj_file* f, int64_t lines) {
+    free_newlines(ctx, f);
+    const int rc = device_alloc(ctx, &f->d_nl, static_cast<size_t>(lines), "cudaMalloc(newline index)");
+    if (!rc) f->nl_cap = lines;
+    return rc;
+}
+
 double now_ms() {
     return std::chrono::duration<double, std::milli>(
                std::chrono::steady_clock::now().time_since_epoch())
         .count();
 }
 
+// A find_value phase from evq0 to here, without waiting for it: it is added
+// to the timings by the next phase's end, whose wait covers it.
+int defer_phase(gpj_ctx* ctx, double host_start) {
+    GPJ_CUDA(ctx, cudaEventRecord(ctx->evq1, ctx->stream));
+    ctx->deferred = true;
+    ctx->deferred_host_ms = now_ms() - host_start;
+    return GPJ_OK;
+}
+
+// Adds the phase between ev0 (recorded at `host_start`) and ev1, both
+// reached, to the timings.
+int close_phase(gpj_ctx* ctx, const char* name, double host_start) {
+    float ms = 0.f;
+    if (ctx->deferred) {
+        ctx->deferred = false;
+        GPJ_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->evq0, ctx->evq1));
+        ctx->phases.push_back(Phase{"find_value", static_cast<double>(ms), ctx->deferred_host_ms});
+    }
+    GPJ_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
+    ctx->phases.push_back(Phase{name, static_cast<double>(ms), now_ms() - host_start});
+    return GPJ_OK;
+}
+
 // Records a phase measured between ev0 (recorded at `host_start`) and now.
 int end_phase(gpj_ctx* ctx, const char* name, double host_start) {
     GPJ_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     GPJ_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
-    float ms = 0.f;
-    GPJ_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-    ctx->phases.push_back(Phase{name, static_cast<double>(ms), now_ms() - host_start});
-    return GPJ_OK;
+    return close_phase(ctx, name, host_start);
 }
 
 int ensure_tile_state(gpj_ctx* ctx, int64_t ntiles) {
@@ -323,13 +380,29 @@ int occupancy_slot(int num_levels) { return num_levels <= 4 ? 0 : (num_levels <=
 // the exact kernel uses the first).
 unsigned int* tile_claims(gpj_ctx* ctx) { return ctx->d_counter + 1; }
 
+// Zeroes the status words, the tile counters and the hand-over count.
+int reset_control(gpj_ctx* ctx) {
+    GPJ_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, kControlBytes, ctx->stream));
+    return GPJ_OK;
+}
+
+// Copies the status words to h_status and waits; ev1 is recorded at the end
+// of the work before them.
+int read_status(gpj_ctx* ctx) {
+    GPJ_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, 2 * sizeof(unsigned long long),
+                                  cudaMemcpyDeviceToHost, ctx->stream));
+    GPJ_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
+    GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return GPJ_OK;
+}
+
 // One launch of an index kernel; on return h_status holds its status words.
 int launch_index(gpj_ctx* ctx, bool exact, const gpj::IndexParams& base) {
     const int64_t ntiles = base.ntiles;
     int rc = ensure_tile_state(ctx, ntiles);
     if (rc) return rc;
-    GPJ_CUDA(ctx, cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned int), ctx->stream));
-    GPJ_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, 2 * sizeof(unsigned long long), ctx->stream));
+    rc = reset_control(ctx);
+    if (rc) return rc;
     gpj::IndexParams p = base;
     p.tile_state = ctx->d_tile_state;
     p.tile_counter = ctx->d_counter;
@@ -341,10 +414,7 @@ int launch_index(gpj_ctx* ctx, bool exact, const gpj::IndexParams& base) {
     GPJ_CUDA(ctx, exact ? gpj::launch_index_kernel(p, static_cast<int>(grid), ctx->stream)
                         : gpj::launch_line_index_kernel(p, static_cast<int>(grid), ctx->stream));
     ctx->launches++;
-    GPJ_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, 2 * sizeof(unsigned long long),
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-    GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return GPJ_OK;
+    return read_status(ctx);
 }
 
 // Maps the error word of an index launch to a status code and message.
@@ -378,19 +448,18 @@ struct TileScratch {
 
 int alloc_tile_scratch(gpj_ctx* ctx, int64_t n, TileScratch* ts) {
     const int64_t ntiles = (n + gpj::kStandaloneTileBytes - 1) / gpj::kStandaloneTileBytes;
-    int rc = device_alloc(ctx, &ts->bits, static_cast<size_t>((n + 63) / 64), "cudaMalloc(newline bitmap)");
-    if (!rc) rc = device_alloc(ctx, &ts->counts, static_cast<size_t>(ntiles), "cudaMalloc(tile counts)");
-    if (!rc)
-        rc = device_alloc(ctx, &ts->offsets, static_cast<size_t>(gpj::newline_offsets_words(ntiles)),
-                          "cudaMalloc(tile offsets)");
-    return rc;
+    const size_t words = static_cast<size_t>((n + 63) / 64);
+    const size_t offsets = static_cast<size_t>(gpj::newline_offsets_words(ntiles));
+    // one allocation: bitmap, offsets, counts
+    const int rc = device_alloc(ctx, &ts->bits, words + offsets + static_cast<size_t>(ntiles + 1) / 2,
+                                "cudaMalloc(newline scratch)");
+    if (rc) return rc;
+    ts->offsets = reinterpret_cast<int64_t*>(ts->bits + words);
+    ts->counts = reinterpret_cast<int32_t*>(ts->offsets + offsets);
+    return GPJ_OK;
 }
 
-void free_tile_scratch(gpj_ctx* ctx, TileScratch* ts) {
-    device_free(ctx, ts->bits);
-    device_free(ctx, ts->counts);
-    device_free(ctx, ts->offsets);
-}
+void free_tile_scratch(gpj_ctx* ctx, TileScratch* ts) { device_free(ctx, ts->bits); }
 
 // Tile states for a build by the standalone kernel over `ntiles` tiles (one
 // epoch for all its launches).
@@ -409,12 +478,12 @@ int tile_ctas_per_sm(const gpj_ctx* ctx, int num_levels) {
     return want > 0 && want < occ ? want : occ;
 }
 
+// (the tile counter is zero before it)
 int launch_tiles(gpj_ctx* ctx, const gpj::IndexParams& base) {
     const int occ = tile_ctas_per_sm(ctx, base.num_levels);
     const int64_t grid = std::min<int64_t>(base.tile_end - base.tile_begin, static_cast<int64_t>(ctx->sms) * occ);
     gpj::IndexParams p = base;
     p.tile_counter = tile_claims(ctx);
-    GPJ_CUDA(ctx, cudaMemsetAsync(p.tile_counter, 0, sizeof(unsigned int), ctx->stream));
     GPJ_CUDA(ctx, gpj::launch_tile_index_kernel(p, static_cast<int>(grid), ctx->stream));
     ctx->launches++;
     return GPJ_OK;
@@ -426,11 +495,8 @@ int finish_tiles(gpj_ctx* ctx, const gpj::IndexParams& p, const TileScratch& ts)
     const int64_t ntiles = (p.n + gpj::kStandaloneTileBytes - 1) / gpj::kStandaloneTileBytes;
     const int64_t grid = std::min<int64_t>((ntiles + 7) / 8, static_cast<int64_t>(ctx->sms) * 8);
     GPJ_CUDA(ctx, gpj::launch_newline_index(p, ts.offsets, static_cast<int>(grid), ctx->stream));
-    ctx->launches += 2;
-    GPJ_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, 2 * sizeof(unsigned long long),
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-    GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return GPJ_OK;
+    ctx->launches += gpj::newline_index_launches(ntiles);
+    return read_status(ctx);
 }
 
 // Builds the index with the line-parallel kernel (evaluating `fq` in the
@@ -443,14 +509,19 @@ int finish_tiles(gpj_ctx* ctx, const gpj::IndexParams& p, const TileScratch& ts)
 // *exact_only (optional, in and out): the input needs the exact kernel (a
 // line kernel flagged it before, so later builds of the same input skip
 // straight to the exact kernel).
+// `grow` (optional): a file with more lines than its newline index d_nl holds
+// gets a larger one (filled from the tiles' bitmaps, without indexing again,
+// unless the exact kernel ran: then *lines tells).
+// On return ev1 is reached.
 int run_index(gpj_ctx* ctx, const uint8_t* d_file, int64_t n, int num_levels, uint64_t* d_str,
               uint64_t* d_lvl, int64_t level_stride, int64_t* d_nl, int64_t nl_cap, int64_t* lines,
               const FusedQueries* fq = nullptr, bool* queries_done = nullptr, uint64_t* d_marks = nullptr, uint32_t* d_odd = nullptr,
-              bool* marks_valid = nullptr, bool* exact_only = nullptr) {
+              bool* marks_valid = nullptr, bool* exact_only = nullptr, gpj_file* grow = nullptr) {
     if (queries_done) *queries_done = false;
     if (marks_valid) *marks_valid = false;
     if (n == 0) {
         if (nl_cap > 0) GPJ_CUDA(ctx, cudaMemsetAsync(d_nl, 0, 8, ctx->stream));
+        GPJ_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
         GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         *lines = 1;
         return GPJ_OK;
@@ -498,10 +569,7 @@ int run_index(gpj_ctx* ctx, const uint8_t* d_file, int64_t n, int num_levels, ui
         // index only: the standalone kernel, then the newline index
         TileScratch ts;
         rc = alloc_tile_scratch(ctx, n, &ts);
-        if (!rc) {
-            const cudaError_t e = cudaMemsetAsync(ctx->d_status, 0, 2 * sizeof(unsigned long long), ctx->stream);
-            if (e != cudaSuccess) rc = cuda_fail(ctx, e, "cudaMemsetAsync(status)");
-        }
+        if (!rc) rc = reset_control(ctx);
         if (!rc) {
             fused.ntiles = (n + gpj::kStandaloneTileBytes - 1) / gpj::kStandaloneTileBytes;  // its own tile size
             fused.tile_end = fused.ntiles;
@@ -513,6 +581,15 @@ int run_index(gpj_ctx* ctx, const uint8_t* d_file, int64_t n, int num_levels, ui
             rc = set_tile_states(ctx, &fused, fused.ntiles);
             if (!rc) rc = launch_tiles(ctx, fused);
             if (!rc) rc = finish_tiles(ctx, fused, ts);
+            const int64_t found = rc ? 0 : static_cast<int64_t>(ctx->h_status[0]);
+            if (grow && found > nl_cap && !(ctx->h_status[1] & (gpj::kErrIrregular | gpj::kFatalErrors))) {
+                rc = resize_newlines(ctx, grow, found);
+                if (!rc) {
+                    fused.newlines = grow->d_nl;
+                    fused.newline_cap = found;
+                    rc = finish_tiles(ctx, fused, ts);
+                }
+            }
         }
         free_tile_scratch(ctx, &ts);
         if (rc) return rc;
@@ -603,8 +680,13 @@ int upload_queries(gpj_ctx* ctx, gpj_file* f, int nq, const uint8_t* const* bc, 
         if (rc) return rc;
         f->d_ir_cap = packed.size() * 2;
     }
+    // (pageable memory: the copy has read it when the call returns; a stream
+    // being captured takes no upload)
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    GPJ_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capturing));
+    f->ir_host.clear();
+    if (capturing != cudaStreamCaptureStatusNone) GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     GPJ_CUDA(ctx, cudaMemcpyAsync(f->d_ir, packed.data(), packed.size(), cudaMemcpyHostToDevice, ctx->stream));
-    GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     f->ir_host.swap(packed);
     return GPJ_OK;
 }
@@ -691,25 +773,28 @@ int ensure_index_buffers(gpj_ctx* ctx, gpj_file* f, int num_levels) {
     int rc;
     if (num_levels < 1 || num_levels > GPJ_MAX_LEVELS)
         return fail(ctx, GPJ_ELIMIT, "Invalid number of levels: " + std::to_string(num_levels));
-    if (!f->d_str && (rc = device_alloc(ctx, &f->d_str, static_cast<size_t>(f->stride), "cudaMalloc(string index)")))
-        return rc;
-    if (!f->d_marks && (rc = device_alloc(ctx, &f->d_marks, static_cast<size_t>(f->stride), "cudaMalloc(key marks)")))
-        return rc;
-    if (!f->d_odd &&
-        (rc = device_alloc(ctx, &f->d_odd, static_cast<size_t>((f->words + 31) / 32), "cudaMalloc(odd words)")))
-        return rc;
+    if (!f->d_str) {
+        // one allocation: string index, key marks, levels, newlines, odd words
+        const int64_t lines = std::min<int64_t>(f->n + 1, f->n / 256 + 1024);
+        rc = device_alloc(ctx, &f->d_str,
+                          static_cast<size_t>((2 + num_levels) * f->stride + lines + (f->words + 63) / 64),
+                          "cudaMalloc(index)");
+        if (rc) return rc;
+        f->d_marks = f->d_str + f->stride;
+        f->d_lvl = f->d_marks + f->stride;
+        f->lvl_cap = num_levels;
+        f->d_nl = reinterpret_cast<int64_t*>(f->d_lvl + num_levels * f->stride);
+        f->nl_cap = lines;
+        f->d_odd = reinterpret_cast<uint32_t*>(f->d_nl + lines);
+        f->lvl_inside = f->nl_inside = true;
+    }
     if (f->lvl_cap < num_levels) {
-        device_free(ctx, f->d_lvl);
-        f->lvl_cap = 0;
+        free_levels(ctx, f);
         rc = device_alloc(ctx, &f->d_lvl, static_cast<size_t>(f->stride) * num_levels, "cudaMalloc(leveled bitmaps)");
         if (rc) return rc;
         f->lvl_cap = num_levels;
     }
-    if (!f->d_nl) {
-        f->nl_cap = std::min<int64_t>(f->n + 1, f->n / 256 + 1024);
-        rc = device_alloc(ctx, &f->d_nl, static_cast<size_t>(f->nl_cap), "cudaMalloc(newline index)");
-        if (rc) return rc;
-    }
+    if (!f->d_nl) return resize_newlines(ctx, f, std::min<int64_t>(f->n + 1, f->n / 256 + 1024));
     return GPJ_OK;
 }
 
@@ -725,18 +810,16 @@ int index_pass(gpj_ctx* ctx, gpj_file* f, int num_levels, const FusedQueries* fq
     GPJ_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     int64_t lines = 0;
     rc = run_index(ctx, f->d_data, f->n, num_levels, f->d_str, f->d_lvl, f->stride, f->d_nl, f->nl_cap, &lines, fq,
-                   queries_done, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only);
+                   queries_done, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only, f);
     if (rc) return rc;
     if (lines > f->nl_cap) {  // more lines than the first guess: size exactly and rebuild
-        device_free(ctx, f->d_nl);
-        f->nl_cap = lines;
-        rc = device_alloc(ctx, &f->d_nl, static_cast<size_t>(lines), "cudaMalloc(newline index)");
+        rc = resize_newlines(ctx, f, lines);
         if (rc) return rc;
         rc = run_index(ctx, f->d_data, f->n, num_levels, f->d_str, f->d_lvl, f->stride, f->d_nl, f->nl_cap, &lines, fq,
-                       queries_done, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only);
+                       queries_done, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only, f);
         if (rc) return rc;
     }
-    rc = end_phase(ctx, fq && fq->nq ? "index_and_query" : "build_index", t0);
+    rc = close_phase(ctx, fq && fq->nq ? "index_and_query" : "build_index", t0);
     if (rc) return rc;
     f->num_lines = lines;
     f->num_levels = num_levels;
@@ -794,7 +877,7 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
             GPJ_CUDA(ctx, cudaMemcpyAsync(f->d_owned, host, static_cast<size_t>(n), cudaMemcpyHostToDevice,
                                           ctx->stream));
         rc = run_index(ctx, f->d_data, n, num_levels, f->d_str, f->d_lvl, f->stride, f->d_nl, f->nl_cap, &lines, nullptr,
-                           nullptr, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only);
+                           nullptr, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only, f);
         if (rc) return rc;
     } else {
         while (!resident && static_cast<int64_t>(ctx->chunk_events.size()) < nchunks) {
@@ -824,7 +907,7 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         if (!rc && cq) rc = device_alloc(ctx, &d_lines, static_cast<size_t>(nchunks + 1), "cudaMalloc(chunk lines)");
         if (!rc) {
             cudaError_t e = cq ? cudaMemsetAsync(d_lines, 0, sizeof(int64_t), ctx->stream) : cudaSuccess;
-            if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_status, 0, 2 * sizeof(unsigned long long), ctx->stream);
+            if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_status, 0, kControlBytes, ctx->stream);
             // the copies start once the buffers exist (pool allocations are ordered on ctx->stream)
             if (e == cudaSuccess && !resident) e = cudaEventRecord(ctx->ev_ready, ctx->stream);
             if (e == cudaSuccess && !resident) e = cudaStreamWaitEvent(ctx->copy_stream, ctx->ev_ready, 0);
@@ -845,6 +928,7 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
             p.tile_end = t1;
             if (!resident)
                 GPJ_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->chunk_events[std::min(k + 1, nchunks - 1)], 0));
+            if (k > 0) GPJ_CUDA(ctx, cudaMemsetAsync(tile_claims(ctx), 0, sizeof(unsigned int), ctx->stream));
             int r = launch_tiles(ctx, p);
             if (r || !cq) return r;
             // the chunk's newline index, then the queries on the lines it completes
@@ -889,7 +973,7 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         if (errs & (gpj::kErrIrregular | gpj::kErrLongLine)) {
             // the whole input is on the device now: index it in one launch (exact fallback inside)
             rc = run_index(ctx, f->d_data, n, num_levels, f->d_str, f->d_lvl, f->stride, f->d_nl, f->nl_cap, &lines, nullptr,
-                           nullptr, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only);
+                           nullptr, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only, f);
             if (rc) return rc;
         } else if ((rc = status_error(ctx, errs))) {
             f->marks_valid = false;
@@ -899,12 +983,10 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         }
     }
     if (lines > f->nl_cap) {  // more lines than the first guess: size exactly and rebuild
-        device_free(ctx, f->d_nl);
-        f->nl_cap = lines;
-        rc = device_alloc(ctx, &f->d_nl, static_cast<size_t>(lines), "cudaMalloc(newline index)");
+        rc = resize_newlines(ctx, f, lines);
         if (rc) return rc;
         rc = run_index(ctx, f->d_data, n, num_levels, f->d_str, f->d_lvl, f->stride, f->d_nl, f->nl_cap, &lines, nullptr,
-                           nullptr, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only);
+                           nullptr, f->d_marks, f->d_odd, &f->marks_valid, &f->exact_only, f);
         if (rc) return rc;
     }
     rc = end_phase(ctx, resident ? "index_and_query" : "load_and_index", t0);
@@ -1120,16 +1202,17 @@ int gpj_create(int device, gpj_ctx** out) {
         if ((e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess)
             return bail(e, "cudaMemPoolSetAttribute");
     }
-    if ((e = cudaMalloc(&ctx->d_counter, 16)) != cudaSuccess) return bail(e, "cudaMalloc(counter)");
     if ((e = cudaMalloc(&ctx->d_long, sizeof(gpj::LongItem) * kLongItems)) != cudaSuccess)
         return bail(e, "cudaMalloc(long lines)");
-    if ((e = cudaMalloc(&ctx->d_long_count, sizeof(unsigned long long))) != cudaSuccess)
-        return bail(e, "cudaMalloc(long line count)");
     ctx->tuning = default_tuning();
-    if ((e = cudaMalloc(&ctx->d_status, 16)) != cudaSuccess) return bail(e, "cudaMalloc(status)");
+    if ((e = cudaMalloc(&ctx->d_status, kControlBytes)) != cudaSuccess) return bail(e, "cudaMalloc(status)");
+    ctx->d_counter = reinterpret_cast<unsigned int*>(ctx->d_status + 2);
+    ctx->d_long_count = ctx->d_status + 3;
     if ((e = cudaMallocHost(&ctx->h_status, 16)) != cudaSuccess) return bail(e, "cudaMallocHost(status)");
     if ((e = cudaEventCreate(&ctx->ev0)) != cudaSuccess) return bail(e, "cudaEventCreate");
     if ((e = cudaEventCreate(&ctx->ev1)) != cudaSuccess) return bail(e, "cudaEventCreate");
+    if ((e = cudaEventCreate(&ctx->evq0)) != cudaSuccess) return bail(e, "cudaEventCreate");
+    if ((e = cudaEventCreate(&ctx->evq1)) != cudaSuccess) return bail(e, "cudaEventCreate");
     const int levels[3] = {4, 8, 16};
     for (int i = 0; i < 3; i++) {
         ctx->index_occupancy[i] = gpj::index_kernel_max_ctas_per_sm(levels[i]);
@@ -1156,9 +1239,7 @@ void gpj_destroy(gpj_ctx* ctx) {
         device_free(ctx, ctx->d_tile_state);
         cudaStreamSynchronize(ctx->own_stream);
     }
-    if (ctx->d_counter) cudaFree(ctx->d_counter);
     if (ctx->d_long) cudaFree(ctx->d_long);
-    if (ctx->d_long_count) cudaFree(ctx->d_long_count);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->copy_stream) {
         cudaStreamSynchronize(ctx->copy_stream);
@@ -1171,6 +1252,9 @@ void gpj_destroy(gpj_ctx* ctx) {
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+    if (ctx->evq0) cudaEventDestroy(ctx->evq0);
+    if (ctx->evq1) cudaEventDestroy(ctx->evq1);
+    if (ctx->h_small) cudaFreeHost(ctx->h_small);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
 }
@@ -1499,11 +1583,9 @@ void gpj_file_release(gpj_file* f) {
     if (f->ctx) {
         gpj_ctx* ctx = f->ctx;
         device_free(ctx, f->d_owned);
+        free_levels(ctx, f);
+        free_newlines(ctx, f);
         device_free(ctx, f->d_str);
-        device_free(ctx, f->d_marks);
-        device_free(ctx, f->d_odd);
-        device_free(ctx, f->d_lvl);
-        device_free(ctx, f->d_nl);
         device_free(ctx, f->d_ir);
         device_free(ctx, f->d_out);
     }
@@ -1583,7 +1665,7 @@ int gpj_build_index_device(gpj_ctx* ctx, const void* d_file, int64_t n, int num_
     rc = run_index(ctx, static_cast<const uint8_t*>(d_file), n, num_levels, d_string_index, d_leveled,
                    (n + 63) / 64, d_newlines, newline_cap, num_lines);
     if (rc) return rc;
-    rc = end_phase(ctx, "build_index", t0);
+    rc = close_phase(ctx, "build_index", t0);
     if (rc) return rc;
     if (*num_lines > newline_cap)
         return fail(ctx, GPJ_ELIMIT, "newline index needs " + std::to_string(*num_lines) + " entries");
@@ -1650,12 +1732,24 @@ static int run_paths(gpj_ctx* ctx, gpj_file* f, int nq, const char* const* paths
         bcs[i] = compiled[i].bytecode.data();
         lens[i] = compiled[i].bytecode.size();
     }
+    if (!(f->indexed && f->num_levels >= depth) && !ctx->fuse_queries &&
+        (ctx->tuning.chunk_tiles <= 0 || f->exact_only || f->n <= kChunkUnit * ctx->tuning.chunk_tiles)) {
+        // the index alone first: then the line count is known, and the
+        // results take no more than they need (the queries are on their way
+        // meanwhile)
+        int needed = 0;
+        rc = upload_queries(ctx, f, nq, bcs.data(), lens.data(), slots, &needed);
+        if (!rc) rc = index_pass(ctx, f, depth, nullptr, nullptr);
+        if (rc) return rc;
+    }
     if (f->indexed && f->num_levels >= depth) {
         // the resident index has enough levels: the queries alone
         rc = ensure_out(ctx, f, static_cast<size_t>(nq) * f->num_lines * slots * 2);
+        const double t0 = now_ms();
+        if (!rc) GPJ_CUDA(ctx, cudaEventRecord(ctx->evq0, ctx->stream));
         if (!rc) rc = query_common(ctx, f, nq, bcs.data(), lens.data(), slots, f->d_out,
                                    static_cast<int64_t>(nq) * f->num_lines * slots * 2, false, nullptr);
-        if (!rc) rc = end_phase(ctx, "find_value", now_ms());
+        if (!rc) rc = defer_phase(ctx, t0);
         if (rc) return rc;
         *slots_out = slots;
         *cap_out = f->num_lines;
@@ -1701,19 +1795,34 @@ int gpj_query_paths(gpj_ctx* ctx, gpj_file* f, int nq, const char* const* paths,
     }
     const double t1 = now_ms();
     cudaEventRecord(ctx->ev0, ctx->stream);
-    for (int q = 0; q < nq; q++) {
-        cudaError_t e = cudaMemcpyAsync(r->offsets + q * per_query, f->d_out + static_cast<size_t>(q) * cap * slots * 2,
-                                        per_query * 8, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e != cudaSuccess) {
-            delete r;
-            return cuda_fail(ctx, e, "cudaMemcpyAsync(results)");
-        }
+    // small results through page-locked memory: one short copy, no staging by the driver
+    const size_t bytes = static_cast<size_t>(nq) * per_query * 8;
+    const bool small = bytes <= kSmallResult && (cap == f->num_lines || nq == 1);
+    if (small && !ctx->h_small && cudaMallocHost(&ctx->h_small, kSmallResult) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->h_small = nullptr;
+    }
+    const bool staged = small && ctx->h_small;
+    cudaError_t e = cudaSuccess;
+    if (cap == f->num_lines || nq == 1) {
+        if (bytes > 0)
+            e = cudaMemcpyAsync(staged ? static_cast<void*>(ctx->h_small) : r->offsets, f->d_out, bytes,
+                                cudaMemcpyDeviceToHost, ctx->stream);
+    } else {
+        for (int q = 0; q < nq && e == cudaSuccess; q++)
+            e = cudaMemcpyAsync(r->offsets + q * per_query, f->d_out + static_cast<size_t>(q) * cap * slots * 2,
+                                per_query * 8, cudaMemcpyDeviceToHost, ctx->stream);
+    }
+    if (e != cudaSuccess) {
+        delete r;
+        return cuda_fail(ctx, e, "cudaMemcpyAsync(results)");
     }
     rc = end_phase(ctx, "copy_results", t1);
     if (rc) {
         delete r;
         return rc;
     }
+    if (staged) std::memcpy(r->offsets, ctx->h_small, bytes);
     *out = r;
     return GPJ_OK;
 }

@@ -116,8 +116,11 @@ int tile_index_max_ctas_per_sm(int num_levels);
 // entries), then every tile's '\n' positions; writes status[0] =
 // newlines + 1 and at most newline_cap entries, and flags kErrIrregular where
 // a tile did not start in the state the tile before it ended in
-// (tile_state).  Two launches, one stream.
+// (tile_state).  One stream.
 cudaError_t launch_newline_index(const IndexParams& p, int64_t* offsets, int grid, cudaStream_t stream);
+// Launches it takes: few tiles' counts are summed up by each warp for itself
+// (1024 tiles: 16 loads a lane, less than the gap between two launches).
+inline int newline_index_launches(int64_t ntiles) { return ntiles <= 1024 ? 1 : 2; }
 // The same for tiles [t0, t1) only, once every earlier tile's newline index
 // is written (t0 and, unless t1 = ntiles, t1 multiples of kNewlineBlockTiles); the number
 // of lines whose both ends are then known goes to device memory

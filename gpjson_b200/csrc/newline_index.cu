@@ -54,16 +54,21 @@ __global__ void __launch_bounds__(kScanThreads) newline_offsets_kernel(const int
 }
 
 // Sum of the tile counts before tile t of the whole batch (all lanes of a
-// warp call it; the block sums are added up by the lanes).
-__device__ __forceinline__ int64_t tiles_before(const int64_t* offsets, int64_t ntiles, int64_t t) {
+// warp call it; the block sums are added up by the lanes).  offsets null:
+// the counts themselves are.
+__device__ __forceinline__ int64_t tiles_before(const int32_t* counts, const int64_t* offsets, int64_t ntiles,
+                                                int64_t t) {
     const int lane = threadIdx.x & 31;
-    const int64_t* block_sums = offsets + ntiles;
-    const int64_t blk = t / kScanThreads;
     int64_t base = 0;
-    for (int64_t b = lane; b < blk; b += 32) base += block_sums[b];
+    if (offsets) {
+        const int64_t blk = t / kScanThreads;
+        for (int64_t b = lane; b < blk; b += 32) base += offsets[ntiles + b];
+    } else {
+        for (int64_t i = lane; i < t; i += 32) base += counts[i];
+    }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) base += __shfl_xor_sync(~0u, base, off);
-    return base + offsets[t];
+    return offsets ? base + offsets[t] : base;
 }
 
 // A warp per tile of [t0, t1): the tile's newlines before it in its file
@@ -94,7 +99,8 @@ __global__ void __launch_bounds__(256) newline_scatter_kernel(const int32_t* cou
             F = files[lo];
         }
         const int64_t lt = t - F.tile_begin;
-        const int64_t base = tiles_before(offsets, ntiles, t) - tiles_before(offsets, ntiles, F.tile_begin);
+        int64_t base = tiles_before(counts, offsets, ntiles, t);
+        if (F.tile_begin > 0) base -= tiles_before(counts, offsets, ntiles, F.tile_begin);
         if (lt == 0 && lane == 0 && F.cap > 0) F.newlines[0] = 0;
         // the start state the tile derived from its first '\n' is the end
         // state of the tile before it (low 48 bits; the rest is a tag)
@@ -163,7 +169,12 @@ cudaError_t launch_newline_index_range(const IndexParams& p, int64_t* offsets, i
 
 cudaError_t launch_newline_index(const IndexParams& p, int64_t* offsets, int grid, cudaStream_t stream) {
     const int64_t ntiles = (p.n + kStandaloneTileBytes - 1) / kStandaloneTileBytes;
-    return launch_newline_index_range(p, offsets, 0, ntiles, nullptr, grid, stream);
+    if (newline_index_launches(ntiles) == 2)
+        return launch_newline_index_range(p, offsets, 0, ntiles, nullptr, grid, stream);
+    const LineFile one{p.newline_bits, (p.n + 63) / 64, p.newlines, p.newline_cap, p.status, 0, ntiles};
+    newline_scatter_kernel<<<grid, 256, 0, stream>>>(p.tile_newlines, nullptr, p.tile_state, ntiles, 0, ntiles, one,
+                                                     nullptr, 0, nullptr);
+    return cudaGetLastError();
 }
 
 }  // namespace gpj
