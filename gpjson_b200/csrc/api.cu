@@ -14,7 +14,9 @@
 #include <atomic>
 #include <chrono>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <thread>
@@ -70,6 +72,16 @@ static gpj_tuning default_tuning() {
     return t;
 }
 
+// Slices a file is read and copied in, how many of them the staging holds
+// (64 MiB), and the most threads that read.  64 MiB from the page cache take
+// 3.9 ms when halves of 32 MiB are read by 16 threads and then copied; in
+// slices of 1 MiB 2.35 ms with 8 threads, 2.45 with 6, 2.8 with 10 and 3.6
+// with 16 (of 16 on the host: the reads then slow the copies down), and 15 %
+// more in slices of 4 MiB.
+static constexpr size_t kStageSlice = 1 << 20;
+static constexpr int kStageSlots = 64;
+static constexpr int64_t kReadThreads = 8;
+
 struct gpj_ctx {
     int device = 0;
     int sms = 0;
@@ -104,9 +116,10 @@ struct gpj_ctx {
     gpj::LongItem* d_long = nullptr;
     unsigned long long* d_long_count = nullptr;
 
-    // pinned staging for file reads
+    // pinned staging for file reads: kStageSlots slices, and the end of the
+    // last copy out of each
     uint8_t* h_stage = nullptr;
-    size_t stage_bytes = 0;
+    cudaEvent_t stage_events[kStageSlots] = {};
 
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // a find_value phase whose end nobody has waited for yet (defer_phase)
@@ -115,6 +128,7 @@ struct gpj_ctx {
     double deferred_host_ms = 0;
     uint8_t* h_small = nullptr;  // pinned, kSmallResult bytes
     int64_t launches = 0;
+    bool counted = false;  // by value_blocks()
     std::vector<Phase> phases;
 };
 
@@ -195,13 +209,136 @@ struct gpj_result {
     }
 };
 
-// Values of a query call gathered on the device (gpj_query_values).
+// Host memory of gathered values: page-locked (copied to at full speed, no
+// page faults) up to kMost in all, free blocks kept for later values of the
+// process until its last context is destroyed.  Larger ones are pageable.
+class ValueBlocks {
+  public:
+    static constexpr size_t kMost = size_t(64) << 20;
+
+    uint8_t* take(size_t size, size_t* cap, bool* pinned) {
+        bool grow = false;  // sizes vary: one that serves the next as well
+        {
+            std::lock_guard<std::mutex> g(mu_);
+            size_t best = free_.size();
+            for (size_t i = 0; i < free_.size(); i++)
+                if (free_[i].second >= size && (best == free_.size() || free_[i].second < free_[best].second)) best = i;
+            if (best < free_.size()) {
+                const auto b = free_[best];
+                free_.erase(free_.begin() + best);
+                *cap = b.second;
+                *pinned = true;
+                return b.first;
+            }
+            grow = !free_.empty();
+        }
+        const size_t want = (size + (grow ? size / 4 : 0) + 0xFFFF) & ~size_t(0xFFFF);
+        void* p = nullptr;
+        *pinned = false;
+        if (reserve(want)) {
+            if (cudaMallocHost(&p, want) == cudaSuccess) {
+                *cap = want;
+                *pinned = true;
+                return static_cast<uint8_t*>(p);
+            }
+            cudaGetLastError();
+            unreserve(want);
+        }
+        *cap = size;
+        p = std::malloc(size);
+        if (p) std::memset(p, 0, size);  // a copy that faults in its own pages is slower
+        return static_cast<uint8_t*>(p);
+    }
+
+    void give(uint8_t* p, size_t cap, bool pinned) {
+        if (!p) return;
+        if (!pinned) {
+            std::free(p);
+            return;
+        }
+        std::lock_guard<std::mutex> g(mu_);
+        try {
+            if (contexts_ > 0) {
+                free_.emplace_back(p, cap);
+                return;
+            }
+        } catch (const std::exception&) {
+            // no room to note it
+        }
+        total_ -= cap;
+        cudaFreeHost(p);
+    }
+
+    void context_created() {
+        std::lock_guard<std::mutex> g(mu_);
+        ++contexts_;
+    }
+    void context_destroyed() {
+        std::lock_guard<std::mutex> g(mu_);
+        if (--contexts_ == 0) drop_free();
+    }
+
+  private:
+    // Room for `size` more page-locked bytes, if need be in place of the free blocks.
+    bool reserve(size_t size) {
+        std::lock_guard<std::mutex> g(mu_);
+        if (total_ + size > kMost) drop_free();
+        if (total_ + size > kMost) return false;
+        total_ += size;
+        return true;
+    }
+    void unreserve(size_t size) {
+        std::lock_guard<std::mutex> g(mu_);
+        total_ -= size;
+    }
+    void drop_free() {
+        for (auto& b : free_) {
+            total_ -= b.second;
+            cudaFreeHost(b.first);
+        }
+        free_.clear();
+    }
+
+    std::mutex mu_;
+    std::vector<std::pair<uint8_t*, size_t>> free_;
+    size_t total_ = 0;  // page-locked bytes, in use or free
+    int contexts_ = 0;
+};
+
+// Never destroyed, so that values released during process exit find it.
+static ValueBlocks& value_blocks() {
+    static ValueBlocks* b = new ValueBlocks;
+    return *b;
+}
+
+// Values of a query call gathered on the device (gpj_query_values), in one block.
 struct gpj_values {
     int64_t nq = 0, lines = 0;
     int slots = 0;
-    std::vector<uint8_t> kinds;     // [nq][lines][slots]
-    std::vector<int64_t> offsets;   // [nq * lines * slots + 1]
-    std::vector<uint8_t> bytes;     // offsets.back() bytes
+    int64_t size = 0;            // bytes of the values
+    int64_t* offsets = nullptr;  // [nq * lines * slots + 1]
+    uint8_t* kinds = nullptr;    // [nq][lines][slots]
+    uint8_t* bytes = nullptr;
+    uint8_t* block = nullptr;
+    size_t cap = 0;
+    bool pinned = false;
+
+    gpj_values() = default;
+    gpj_values(const gpj_values&) = delete;
+    gpj_values& operator=(const gpj_values&) = delete;
+    ~gpj_values() { value_blocks().give(block, cap, pinned); }
+
+    bool allocate(int64_t items, int64_t total) {
+        const size_t at_kinds = static_cast<size_t>(items + 1) * 8;
+        const size_t at_bytes = (at_kinds + static_cast<size_t>(items) + 15) & ~size_t(15);
+        block = value_blocks().take(at_bytes + static_cast<size_t>(total) + 16, &cap, &pinned);
+        if (!block) return false;
+        offsets = reinterpret_cast<int64_t*>(block);
+        kinds = block + at_kinds;
+        bytes = block + at_bytes;
+        size = total;
+        return true;
+    }
 };
 
 // Requests (file, paths) evaluated together by gpj_batch_run.
@@ -1117,7 +1254,8 @@ int ensure_out(gpj_ctx* ctx, gpj_file* f, size_t elems) {
 // Value extraction over result pairs of file f (values.cu): kinds and
 // offsets, then (d_bytes_out given) a device buffer of exactly the total is
 // allocated into *d_bytes_out, else the values go into d_bytes (cap bytes;
-// null when cap is 0).  *total receives the byte total; synchronous.
+// null when cap is 0).  *total receives the byte total; synchronous, but for
+// the copy of the values with d_bytes_out.
 int gather_values(gpj_ctx* ctx, gpj_file* f, const int64_t* d_pairs, int64_t npairs, int64_t per_query,
                   int64_t stride, uint8_t* d_kinds, int64_t* d_offsets, uint8_t* d_bytes, int64_t cap,
                   uint8_t** d_bytes_out, int64_t* total) {
@@ -1145,6 +1283,7 @@ int gather_values(gpj_ctx* ctx, gpj_file* f, const int64_t* d_pairs, int64_t npa
                                              d_kinds, d_offsets, scratch, d_total, d_bytes, cap, static_cast<int>(grid),
                                              ctx->stream));
         ctx->launches++;
+        if (d_bytes_out) return GPJ_OK;  // the total is known
         GPJ_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, d_total, 8, cudaMemcpyDeviceToHost, ctx->stream));
         GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         *total = static_cast<int64_t>(ctx->h_status[0]);
@@ -1226,6 +1365,8 @@ int gpj_create(int device, gpj_ctx** out) {
         ctx->query_occupancy[v] = gpj::find_value_max_ctas_per_sm(v == 0 ? 4 : (v == 1 ? 8 : GPJ_MAX_LEVELS));
         if (ctx->query_occupancy[v] < 1) return bail(cudaGetLastError(), "find_value occupancy");
     }
+    value_blocks().context_created();
+    ctx->counted = true;
     *out = ctx;
     return GPJ_OK;
 }
@@ -1233,6 +1374,7 @@ int gpj_create(int device, gpj_ctx** out) {
 void gpj_destroy(gpj_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
+    if (ctx->counted) value_blocks().context_destroyed();
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->own_stream) {
         ctx->stream = ctx->own_stream;
@@ -1250,6 +1392,8 @@ void gpj_destroy(gpj_ctx* ctx) {
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+    for (cudaEvent_t e : ctx->stage_events)
+        if (e) cudaEventDestroy(e);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->evq0) cudaEventDestroy(ctx->evq0);
@@ -1513,59 +1657,62 @@ int gpj_file_open(gpj_ctx* ctx, const char* filename, gpj_file** out) {
         return rc;
     }
     f->d_data = f->d_owned;
-    // Two pinned halves: the read of one chunk overlaps the copy of the other.
-    const size_t chunk = 32u << 20;
     if (!ctx->h_stage) {
-        cudaError_t e = cudaMallocHost(&ctx->h_stage, 2 * chunk);
+        cudaError_t e = cudaMallocHost(&ctx->h_stage, kStageSlice * kStageSlots);
         if (e != cudaSuccess) {
+            ctx->h_stage = nullptr;
             ::close(fd);
             gpj_file_release(f);
             return cuda_fail(ctx, e, "cudaMallocHost(staging)");
         }
-        ctx->stage_bytes = 2 * chunk;
     }
-    // one reader thread per 2 MiB of a chunk, at most one per host thread (and 16)
+    cudaError_t ce = cudaSuccess;
+    for (cudaEvent_t& e : ctx->stage_events)
+        if (!e && ce == cudaSuccess) ce = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    rc = ce == cudaSuccess ? GPJ_OK : cuda_fail(ctx, ce, "cudaEventCreate(file slices)");
+    // one thread per 2 MiB, at most one per host thread (and kReadThreads)
     const int threads = static_cast<int>(std::min<int64_t>(
-        std::min<int64_t>(16, std::max(1u, std::thread::hardware_concurrency())), std::max<int64_t>(1, n >> 21)));
+        std::min<int64_t>(kReadThreads, std::max(1u, std::thread::hardware_concurrency())),
+        std::max<int64_t>(1, n >> 21)));
     const double t0 = now_ms();
     cudaEventRecord(ctx->ev0, ctx->stream);
-    // done[h]: the copy out of staging half h has finished (a half is
-    // refilled only after that)
-    cudaEvent_t done[2] = {nullptr, nullptr};
-    cudaError_t ce = cudaEventCreateWithFlags(&done[0], cudaEventDisableTiming);
-    if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&done[1], cudaEventDisableTiming);
-    rc = ce == cudaSuccess ? GPJ_OK : cuda_fail(ctx, ce, "cudaEventCreate(file chunks)");
     if (!rc) {
+        // Each thread reads a slice into its slot of the staging and queues
+        // its copy, so the reads go on while earlier slices are copied.
         gpj::SliceReader reader(fd, threads);
-        int64_t pos = 0;
-        int half = 0;
-        while (pos < n) {
-            const size_t want = static_cast<size_t>(std::min<int64_t>(static_cast<int64_t>(chunk), n - pos));
-            uint8_t* stage = ctx->h_stage + half * chunk;
-            cudaError_t e = cudaEventSynchronize(done[half]);
-            if (e != cudaSuccess) {
-                rc = cuda_fail(ctx, e, "cudaEventSynchronize(file chunk)");
-                break;
+        std::atomic<int> copy_error{cudaSuccess};
+        std::atomic<int64_t> queued[kStageSlots] = {};  // per slot: the last slice whose copy its event ends, + 1
+        const bool ok = reader.for_each((n + static_cast<int64_t>(kStageSlice) - 1) / static_cast<int64_t>(kStageSlice),
+                                        [&](int64_t i) {
+            const int slot = static_cast<int>(i % kStageSlots);
+            const int64_t pos = i * static_cast<int64_t>(kStageSlice);
+            const size_t want = static_cast<size_t>(std::min<int64_t>(static_cast<int64_t>(kStageSlice), n - pos));
+            uint8_t* stage = ctx->h_stage + slot * kStageSlice;
+            cudaError_t e = cudaSetDevice(ctx->device);
+            if (e == cudaSuccess && i >= kStageSlots) {
+                // the slot's last slice (taken earlier, so some thread is at it) has left it
+                while (queued[slot].load(std::memory_order_acquire) != i - kStageSlots + 1) {
+                    if (reader.failed()) return false;
+                    std::this_thread::yield();
+                }
+                e = cudaEventSynchronize(ctx->stage_events[slot]);
             }
-            if (!reader.read(stage, pos, want)) {
-                rc = fail(ctx, GPJ_EIO, std::string("Size of file has changed while reading ") + filename);
-                break;
-            }
-            e = cudaMemcpyAsync(f->d_owned + pos, stage, want, cudaMemcpyHostToDevice, ctx->stream);
-            if (e == cudaSuccess) e = cudaEventRecord(done[half], ctx->stream);
-            if (e != cudaSuccess) {
-                rc = cuda_fail(ctx, e, "cudaMemcpyAsync(file)");
-                break;
-            }
-            pos += static_cast<int64_t>(want);
-            half ^= 1;
-        }
+            if (e == cudaSuccess && !reader.read_here(stage, pos, want)) return false;
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(f->d_owned + pos, stage, want, cudaMemcpyHostToDevice, ctx->stream);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->stage_events[slot], ctx->stream);
+            queued[slot].store(i + 1, std::memory_order_release);
+            if (e != cudaSuccess) copy_error = e;
+            return e == cudaSuccess;
+        });
+        if (copy_error != cudaSuccess)
+            rc = cuda_fail(ctx, static_cast<cudaError_t>(copy_error.load()), "cudaMemcpyAsync(file)");
+        else if (!ok)
+            rc = fail(ctx, GPJ_EIO, std::string("Size of file has changed while reading ") + filename);
     }
     ::close(fd);
     if (rc == GPJ_OK) rc = end_phase(ctx, "read_file", t0);
     else cudaStreamSynchronize(ctx->stream);  // no copy still reads the staging
-    if (done[0]) cudaEventDestroy(done[0]);
-    if (done[1]) cudaEventDestroy(done[1]);
     if (rc) {
         gpj_file_release(f);
         return rc;
@@ -1881,27 +2028,21 @@ int gpj_query_values(gpj_ctx* ctx, gpj_file* f, int nq, const char* const* paths
     if (!rc)
         rc = gather_values(ctx, f, f->d_out, npairs, per_query, cap * slots, d_kinds, d_offsets, nullptr, 0, &d_bytes,
                            &total);
-    if (!rc) {
-        try {
-            v->kinds.resize(static_cast<size_t>(npairs));
-            v->offsets.resize(static_cast<size_t>(npairs + 1));
-            v->bytes.resize(static_cast<size_t>(total));
-        } catch (const std::bad_alloc&) {
-            rc = fail(ctx, GPJ_ENOMEM, "out of host memory for values");
-        }
-    }
+    if (!rc && !v->allocate(npairs, total)) rc = fail(ctx, GPJ_ENOMEM, "out of host memory for values");
     cudaError_t e = cudaSuccess;
-    if (!rc && npairs > 0) e = cudaMemcpyAsync(v->kinds.data(), d_kinds, npairs, cudaMemcpyDeviceToHost, ctx->stream);
+    if (!rc && npairs > 0) e = cudaMemcpyAsync(v->kinds, d_kinds, npairs, cudaMemcpyDeviceToHost, ctx->stream);
     if (!rc && e == cudaSuccess)
-        e = cudaMemcpyAsync(v->offsets.data(), d_offsets, (npairs + 1) * 8, cudaMemcpyDeviceToHost, ctx->stream);
+        e = cudaMemcpyAsync(v->offsets, d_offsets, (npairs + 1) * 8, cudaMemcpyDeviceToHost, ctx->stream);
     if (!rc && e == cudaSuccess && total > 0)
-        e = cudaMemcpyAsync(v->bytes.data(), d_bytes, total, cudaMemcpyDeviceToHost, ctx->stream);
-    if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        e = cudaMemcpyAsync(v->bytes, d_bytes, total, cudaMemcpyDeviceToHost, ctx->stream);
     if (!rc && e != cudaSuccess) rc = cuda_fail(ctx, e, "copy of values");
     device_free(ctx, d_kinds);
     device_free(ctx, d_offsets);
     device_free(ctx, d_bytes);
-    if (!rc) rc = end_phase(ctx, "gather_values", t0);
+    if (!rc)
+        rc = end_phase(ctx, "gather_values", t0);
+    else
+        cudaStreamSynchronize(ctx->stream);  // no copy still writes the block
     if (rc) {
         delete v;
         return rc;
@@ -1913,10 +2054,10 @@ int gpj_query_values(gpj_ctx* ctx, gpj_file* f, int nq, const char* const* paths
 int64_t gpj_values_num_queries(const gpj_values* v) { return v ? v->nq : 0; }
 int64_t gpj_values_num_lines(const gpj_values* v) { return v ? v->lines : 0; }
 int gpj_values_slots(const gpj_values* v) { return v ? v->slots : 0; }
-const uint8_t* gpj_values_kinds(const gpj_values* v) { return v ? v->kinds.data() : nullptr; }
-const int64_t* gpj_values_offsets(const gpj_values* v) { return v ? v->offsets.data() : nullptr; }
-const uint8_t* gpj_values_bytes(const gpj_values* v) { return v ? v->bytes.data() : nullptr; }
-int64_t gpj_values_size(const gpj_values* v) { return v ? static_cast<int64_t>(v->bytes.size()) : 0; }
+const uint8_t* gpj_values_kinds(const gpj_values* v) { return v ? v->kinds : nullptr; }
+const int64_t* gpj_values_offsets(const gpj_values* v) { return v ? v->offsets : nullptr; }
+const uint8_t* gpj_values_bytes(const gpj_values* v) { return v ? v->bytes : nullptr; }
+int64_t gpj_values_size(const gpj_values* v) { return v ? v->size : 0; }
 void gpj_values_release(gpj_values* v) { delete v; }
 
 int gpj_get_timings(gpj_ctx* ctx, char* json, size_t cap, size_t* len) {

@@ -8,6 +8,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cerrno>
 #include <condition_variable>
 #include <cstdint>
@@ -19,21 +20,18 @@
 
 namespace gpj {
 
-// Reads byte ranges of a file into host memory with up to `threads`
-// threads: each range is cut into one slice per thread, read concurrently
-// by preads.  A file load is bound by this copy out of the page cache,
-// which one thread does at a fraction of host memory bandwidth.  The
-// workers live for one load, so a range costs two condition-variable
-// round trips, not thread starts.
+// Reads a file with up to `threads` threads, the caller's among them.  A
+// file load is bound by the copy out of the page cache, which one thread
+// does at a fraction of host memory bandwidth.  The workers live for one
+// load.
 class SliceReader {
   public:
     SliceReader(int fd, int threads) : fd_(fd) {
         try {
-            for (int i = 1; i < threads; i++) workers_.emplace_back([this, i] { work(i); });
+            for (int i = 1; i < threads; i++) workers_.emplace_back([this] { work(); });
         } catch (const std::exception&) {
-            // fewer threads than asked: the ranges are cut into fewer slices
+            // fewer threads than asked
         }
-        parts_ = static_cast<int>(workers_.size()) + 1;
     }
 
     ~SliceReader() {
@@ -45,34 +43,44 @@ class SliceReader {
         for (auto& t : workers_) t.join();
     }
 
-    // Bytes [pos, pos + len) into dst; false on an I/O error or a short
-    // read (the file shrank).
-    bool read(uint8_t* dst, int64_t pos, size_t len) {
+    // Calls fn(i) once for each i in [0, count), numbers taken in order by
+    // whichever thread is free; false when one of them returned false (no
+    // more are taken then).
+    template <class Fn>
+    bool for_each(int64_t count, const Fn& fn) {
         {
             std::lock_guard<std::mutex> g(mu_);
-            dst_ = dst;
-            pos_ = pos;
-            len_ = len;
+            fn_ = &fn;
+            call_ = [](const void* f, int64_t i) { return (*static_cast<const Fn*>(f))(i); };
+            count_ = count;
+            next_ = 0;
             ok_ = true;
-            pending_ = parts_ - 1;
+            pending_ = static_cast<int>(workers_.size());
             ++round_;
         }
         go_.notify_all();
-        const bool mine = read_slice(0);
+        take();
         std::unique_lock<std::mutex> g(mu_);
         done_.wait(g, [this] { return pending_ == 0; });
-        return mine && ok_;
+        return ok_;
     }
 
-  private:
-    // Slice i of the current range (the range is fixed until every slice is read).
-    bool read_slice(int i) const {
-        const size_t slice = (len_ + parts_ - 1) / parts_;
-        const size_t off = std::min(len_, slice * static_cast<size_t>(i));
-        const size_t want = std::min(slice, len_ - off);
+    // Bytes [pos, pos + len) into dst, a slice per thread; false on an I/O
+    // error or a short read (the file shrank).
+    bool read(uint8_t* dst, int64_t pos, size_t len) {
+        const size_t parts = workers_.size() + 1;
+        const size_t slice = (len + parts - 1) / parts;
+        return for_each(static_cast<int64_t>(parts), [&](int64_t i) {
+            const size_t off = std::min(len, slice * static_cast<size_t>(i));
+            return read_here(dst + off, pos + static_cast<int64_t>(off), std::min(slice, len - off));
+        });
+    }
+
+    // The same on the calling thread alone (from any thread).
+    bool read_here(uint8_t* dst, int64_t pos, size_t len) const {
         size_t got = 0;
-        while (got < want) {
-            const ssize_t r = ::pread(fd_, dst_ + off + got, want - got, static_cast<off_t>(pos_ + off + got));
+        while (got < len) {
+            const ssize_t r = ::pread(fd_, dst + got, len - got, static_cast<off_t>(pos + got));
             if (r < 0 && errno == EINTR) continue;
             if (r <= 0) return false;
             got += static_cast<size_t>(r);
@@ -80,7 +88,15 @@ class SliceReader {
         return true;
     }
 
-    void work(int i) {
+    bool failed() const { return !ok_; }
+
+  private:
+    void take() {
+        for (int64_t i = next_++; i < count_ && ok_; i = next_++)
+            if (!call_(fn_, i)) ok_ = false;
+    }
+
+    void work() {
         uint64_t seen = 0;
         for (;;) {
             {
@@ -89,10 +105,9 @@ class SliceReader {
                 if (quit_) return;
                 seen = round_;
             }
-            const bool ok = read_slice(i);
+            take();
             {
                 std::lock_guard<std::mutex> g(mu_);
-                ok_ = ok_ && ok;
                 --pending_;
             }
             done_.notify_one();
@@ -100,16 +115,18 @@ class SliceReader {
     }
 
     const int fd_;
-    int parts_ = 1;
     std::vector<std::thread> workers_;
     std::mutex mu_;
     std::condition_variable go_, done_;
     uint64_t round_ = 0;
     int pending_ = 0;
-    bool ok_ = true, quit_ = false;
-    uint8_t* dst_ = nullptr;
-    int64_t pos_ = 0;
-    size_t len_ = 0;
+    bool quit_ = false;
+    // the current call of for_each
+    const void* fn_ = nullptr;
+    bool (*call_)(const void*, int64_t) = nullptr;
+    int64_t count_ = 0;
+    std::atomic<int64_t> next_{0};
+    std::atomic<bool> ok_{true};
 };
 
 // Host memory for results.  A new buffer's first touch (page faults) costs
