@@ -57,6 +57,14 @@ static constexpr int64_t kLongLineBytes = 8192;
 static constexpr int64_t kFewPairs = 1 << 13;
 static constexpr int64_t kFewBatchPairs = 4096;
 
+// Results of a batch (int64 numbers, 8 MiB) evaluated by one launch at the
+// least; the next launch runs while they are copied to the host.  48 files,
+// 734 MiB, 44 MB of results: 1358 us in one launch and one copy after it, 920
+// in groups of 4 or 8 MiB, 1050 of 16, 1100 of 2 (the ends of the launches
+// add up), 1100 of 8 when the files with long lines are in several groups,
+// 1620 when the kernel writes the results to the host's memory itself.
+static constexpr size_t kGroupOut = size_t(8) << 17;
+
 // gpj_ctx::d_status and what follows it.
 static constexpr size_t kControlBytes = 32;
 
@@ -341,6 +349,16 @@ struct gpj_values {
     }
 };
 
+// Consecutive files of a batch that one launch evaluates.
+struct BatchGroup {
+    size_t first = 0;                     // file, in the order they are evaluated
+    size_t out_begin = 0, out_end = 0;    // results (int64 numbers)
+    int files = 0, depth = 0;
+    int64_t items = 0, warp_items = 0;
+
+    BatchGroup(size_t file, size_t out) : first(file), out_begin(out), out_end(out) {}
+};
+
 // Requests (file, paths) evaluated together by gpj_batch_run.
 struct gpj_batch {
     gpj_ctx* ctx = nullptr;
@@ -356,6 +374,7 @@ struct gpj_batch {
         int depth = 0, slots = 1;
         int64_t lines = 0;
         bool by_warp = false;   // its lines a warp each
+        int64_t item_begin = 0, warp_begin = 0;  // in its group's launch
         size_t out_offset = 0;  // elements into `results`
     };
     std::vector<Item> items;
@@ -2295,11 +2314,31 @@ int gpj_batch_run(gpj_batch* b) {
     // one find_value launch over every line of every file
     const double t0 = now_ms();
     GPJ_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
+    // Files whose lines are long, or all when the batch is small, have their
+    // lines evaluated a warp each.  They come last: their results are few,
+    // and their launch, as long as its longest lines take, runs while those
+    // of the others are copied.
+    int64_t pairs = 0;
+    for (auto& fr : b->files) {
+        fr.lines = fr.file->num_lines;
+        pairs += fr.lines * static_cast<int64_t>(fr.queries.size());
+    }
+    std::vector<size_t> order;
+    for (size_t i = 0; i < b->files.size(); i++) {
+        auto& fr = b->files[i];
+        fr.by_warp = ctx->tuning.long_line_bytes >= 0 &&
+                     (pairs <= kFewBatchPairs ||
+                      gpj::query_by_warp(fr.lines, fr.file->n, static_cast<int>(fr.queries.size()), 0));
+        if (!fr.by_warp) order.push_back(i);
+    }
+    for (size_t i = 0; i < b->files.size(); i++)
+        if (b->files[i].by_warp) order.push_back(i);
     std::vector<uint8_t> blob;  // per file: [int32 offsets (16-byte padded)][programs]
     std::vector<size_t> blob_at(b->files.size());
+    std::vector<BatchGroup> groups;
     size_t total_out = 0;
-    int64_t total_items = 0, warp_items = 0, pairs = 0;
-    for (size_t i = 0; i < b->files.size(); i++) {
+    for (size_t k = 0; k < order.size(); k++) {
+        const size_t i = order[k];
         auto& fr = b->files[i];
         const size_t nq = fr.queries.size();
         blob_at[i] = blob.size();
@@ -2310,30 +2349,30 @@ int gpj_batch_run(gpj_batch* b) {
             std::memcpy(blob.data() + blob_at[i] + 4 * q, &off, 4);
         }
         blob.resize((blob.size() + 15) / 16 * 16, 0);
-        fr.lines = fr.file->num_lines;
+        if (groups.empty() || total_out - groups.back().out_begin >= kGroupOut ||
+            (groups.size() > 1 && fr.by_warp && !b->files[order[k - 1]].by_warp))
+            groups.push_back(BatchGroup{k, total_out});
+        BatchGroup& gr = groups.back();
         fr.out_offset = total_out;
-        total_out += nq * static_cast<size_t>(fr.lines) * fr.slots * 2;
-        pairs += fr.lines * static_cast<int64_t>(nq);
-    }
-    // Files whose lines are long, or all when the batch is small, have their
-    // lines evaluated a warp each.
-    for (auto& fr : b->files) {
-        const int nq = static_cast<int>(fr.queries.size());
-        fr.by_warp = ctx->tuning.long_line_bytes >= 0 &&
-                     (pairs <= kFewBatchPairs || gpj::query_by_warp(fr.lines, fr.file->n, nq, 0));
+        fr.item_begin = gr.items;
+        fr.warp_begin = gr.warp_items;
         if (fr.by_warp)
-            warp_items += fr.lines * nq;
+            gr.warp_items += fr.lines * static_cast<int64_t>(nq);
         else
-            total_items += gpj::query_items(fr.lines, nq);
+            gr.items += gpj::query_items(fr.lines, static_cast<int>(nq));
+        gr.depth = std::max(gr.depth, fr.depth);
+        gr.files++;
+        total_out += nq * static_cast<size_t>(fr.lines) * fr.slots * 2;
+        gr.out_end = total_out;
     }
-    const int launches = (total_items > 0 ? 1 : 0) +
-                         (warp_items > 0 || (total_items > 0 && long_lines(ctx).items) ? 1 : 0);
+    int launches = 0;
+    for (const BatchGroup& gr : groups)
+        launches += (gr.items > 0 ? 1 : 0) +
+                    (gr.warp_items > 0 || (gr.items > 0 && long_lines(ctx).items) ? 1 : 0);
     // what the query phase reads: replay its graph when nothing of it changed
-    int depth = 0;
-    for (auto& fr : b->files) depth = std::max(depth, fr.depth);
     std::vector<uint64_t> sig{static_cast<uint64_t>(reinterpret_cast<uintptr_t>(ctx->stream)),
-                              static_cast<uint64_t>(ctx->tuning.long_line_bytes),
-                              static_cast<uint64_t>(query_occupancy(ctx, depth))};
+                              static_cast<uint64_t>(ctx->tuning.long_line_bytes)};
+    for (const BatchGroup& gr : groups) sig.push_back(static_cast<uint64_t>(query_occupancy(ctx, gr.depth)));
     for (auto& fr : b->files) {
         gpj_file* f = fr.file;
         for (uint64_t v : {static_cast<uint64_t>(reinterpret_cast<uintptr_t>(f)),
@@ -2371,9 +2410,8 @@ int gpj_batch_run(gpj_batch* b) {
     if (!rc) rc = device_alloc(ctx, &d_qf, b->files.size(), "cudaMalloc(batch query files)");
     bool captured = false;
     if (!rc) {
-        std::vector<gpj::QueryFile> qf;
-        int64_t item = 0, warp_item = 0;
-        for (size_t i = 0; i < b->files.size(); i++) {
+        std::vector<gpj::QueryFile> qf;  // in `order`
+        for (const size_t i : order) {
             auto& fr = b->files[i];
             gpj_file* f = fr.file;
             const size_t nq = fr.queries.size();
@@ -2381,13 +2419,9 @@ int gpj_batch_run(gpj_batch* b) {
             qf.push_back(gpj::QueryFile{f->d_data, f->n, f->d_nl, fr.lines, f->d_str, f->d_lvl, f->stride,
                                         d_blob + blob_at[i] + header,
                                         reinterpret_cast<const int32_t*>(d_blob + blob_at[i]),
-                                        static_cast<int>(nq), fr.slots, d_out + fr.out_offset, fr.lines, item,
+                                        static_cast<int>(nq), fr.slots, d_out + fr.out_offset, fr.lines, fr.item_begin,
                                         f->marks_valid ? f->d_marks : nullptr,
-                                        f->marks_valid ? f->d_odd : nullptr, warp_item});
-            if (fr.by_warp)
-                warp_item += fr.lines * static_cast<int64_t>(nq);
-            else
-                item += gpj::query_items(fr.lines, static_cast<int>(nq));
+                                        f->marks_valid ? f->d_odd : nullptr, fr.warp_begin});
         }
         cudaError_t e = cudaMemcpyAsync(d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess)
@@ -2426,19 +2460,33 @@ int gpj_batch_run(gpj_batch* b) {
         if (pick) b->cur = pick;
         // the query phase: captured as a graph (kept for the next run) when
         // the stream allows it, else launched directly
-        const int64_t grid = std::max<int64_t>(
-            1, std::min<int64_t>((total_items + gpj::kQueryThreads - 1) / gpj::kQueryThreads,
-                                 static_cast<int64_t>(ctx->sms) * query_occupancy(ctx, depth)));
         auto query_phase = [&]() -> cudaError_t {
             cudaError_t q = cudaSuccess;
-            const gpj::LongLines ll = total_items > 0 ? long_lines(ctx) : gpj::LongLines{};
-            if (ll.items) q = cudaMemsetAsync(ctx->d_long_count, 0, sizeof(unsigned long long), ctx->stream);
-            if (q == cudaSuccess)
-                q = gpj::launch_find_value_batch(d_qf, static_cast<int>(qf.size()), total_items, warp_items, depth, ll,
-                                                 static_cast<int>(grid), warp_grid(ctx, warp_items, ll.items != nullptr),
-                                                 ctx->stream);
-            if (q == cudaSuccess && total_out > 0)
-                q = cudaMemcpyAsync(pick->p, d_out, total_out * 8, cudaMemcpyDeviceToHost, ctx->stream);
+            for (const BatchGroup& gr : groups) {
+                const gpj::LongLines ll = gr.items > 0 ? long_lines(ctx) : gpj::LongLines{};
+                const int64_t grid = std::max<int64_t>(
+                    1, std::min<int64_t>((gr.items + gpj::kQueryThreads - 1) / gpj::kQueryThreads,
+                                         static_cast<int64_t>(ctx->sms) * query_occupancy(ctx, gr.depth)));
+                if (ll.items) q = cudaMemsetAsync(ctx->d_long_count, 0, sizeof(unsigned long long), ctx->stream);
+                if (q == cudaSuccess)
+                    q = gpj::launch_find_value_batch(d_qf + gr.first, gr.files, gr.items, gr.warp_items, gr.depth, ll,
+                                                     static_cast<int>(grid),
+                                                     warp_grid(ctx, gr.warp_items, ll.items != nullptr), ctx->stream);
+                // the last group's results follow on the stream itself
+                const bool last = &gr == &groups.back();
+                cudaStream_t to = last ? ctx->stream : ctx->copy_stream;
+                if (!last && q == cudaSuccess) q = cudaEventRecord(ctx->ev_ready, ctx->stream);
+                if (!last && q == cudaSuccess) q = cudaStreamWaitEvent(to, ctx->ev_ready, 0);
+                if (q == cudaSuccess && gr.out_end > gr.out_begin)
+                    q = cudaMemcpyAsync(pick->p + gr.out_begin, d_out + gr.out_begin, (gr.out_end - gr.out_begin) * 8,
+                                        cudaMemcpyDeviceToHost, to);
+                if (q != cudaSuccess) break;
+            }
+            if (groups.size() > 1) {  // also after an error: the copies have ended when the stream has
+                cudaError_t j = cudaEventRecord(ctx->ev_ready, ctx->copy_stream);
+                if (j == cudaSuccess) j = cudaStreamWaitEvent(ctx->stream, ctx->ev_ready, 0);
+                if (q == cudaSuccess) q = j;
+            }
             return q;
         };
         cudaGraphExec_t exec = nullptr;
@@ -2462,8 +2510,11 @@ int gpj_batch_run(gpj_batch* b) {
             e = captured ? cudaGraphLaunch(exec, ctx->stream) : query_phase();
         }
         ctx->launches += launches;
-        if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        if (!rc && e != cudaSuccess) rc = cuda_fail(ctx, e, "batch query");
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(ctx->stream);
+        else
+            cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) rc = cuda_fail(ctx, e, "batch query");
         if (captured && !rc) {
             b->replay.exec = exec;
             b->replay.sig = sig;
