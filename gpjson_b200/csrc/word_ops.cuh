@@ -342,6 +342,12 @@ GPJ_HD bool split_range_ok(int depth, int opens, int closes) {
     return depth + opens < 2 * LV - 1 && depth - closes >= -LV;
 }
 
+// No byte of the half is at a level below LV (it has none to mark).
+template <int LV>
+GPJ_HD bool split_above(int depth, int closes) {
+    return depth - closes >= LV;
+}
+
 template <int LV>
 GPJ_HD void split_half(uint32_t open, uint32_t close, uint32_t structural, int depth, uint32_t (&lv)[LV],
                        uint32_t& at_minus_one) {

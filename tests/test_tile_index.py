@@ -114,3 +114,30 @@ def test_tile_edges(gpjson, levels):
                 assert np.array_equal(f.leveled_bitmaps(levels), want.levels), name
         finally:
             f.release()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("levels", [1, 4, 7, 8, 12, 16])
+def test_levels_above_the_marked_ones(gpjson, levels):
+    """Lines whose nesting wanders around and far above the marked levels."""
+    r = random.Random(levels)
+    lines = []
+    for _ in range(400):
+        depth, top, line = 0, r.choice([3, levels, levels + 3, 2 * levels + 9, 200]), []
+        for _ in range(r.choice([10, 100, 3000])):
+            up = r.random() < (0.7 if depth < top else 0.3)
+            line.append(r.choice(["[", "{", ",[", ', "[:]", {']) if up or depth == 0 else r.choice(["]", "}", ",]", " ] "]))
+            depth += 1 if up or depth == 0 else -1
+            if r.random() < 0.3:
+                line.append(r.choice([",", ":", " " * r.randint(1, 90)]))
+        lines.append("".join(line) + "]" * depth)
+    data = "\n".join(lines).encode()
+    want = oracle.Index(data, levels)
+    f = gpjson.load_bytes(data)
+    try:
+        f.build_index(levels)
+        assert np.array_equal(f.newline_index(), want.newlines)
+        assert np.array_equal(f.string_index(), want.strings)
+        assert np.array_equal(f.leveled_bitmaps(levels), want.levels)
+    finally:
+        f.release()
