@@ -65,6 +65,10 @@ static constexpr int64_t kFewBatchPairs = 4096;
 // 1620 when the kernel writes the results to the host's memory itself.
 static constexpr size_t kGroupOut = size_t(8) << 17;
 
+// Inputs from this size on have their index in several allocations: an
+// allocation takes 2 us, a pass over them 100 and more.
+static constexpr int64_t kApartBytes = int64_t(128) << 20;
+
 // gpj_ctx::d_status and what follows it.
 static constexpr size_t kControlBytes = 32;
 
@@ -151,7 +155,7 @@ struct gpj_file {
     int64_t stride = 0;
 
     uint64_t* d_str = nullptr;
-    // for find_value's key searches (IndexParams::marks, odd), after d_str in its allocation
+    // for find_value's key searches (IndexParams::marks, odd)
     uint64_t* d_marks = nullptr;
     uint32_t* d_odd = nullptr;
     bool marks_valid = false;  // they belong to the current index
@@ -161,6 +165,7 @@ struct gpj_file {
     int64_t nl_cap = 0;
     // they lie in d_str's allocation (until more levels or lines are needed)
     bool lvl_inside = false, nl_inside = false;
+    bool apart = false;  // each part has an allocation of its own
     bool indexed = false;
     bool exact_only = false;  // the line kernels flagged this input: index it with the exact kernel
     int num_levels = 0;
@@ -930,19 +935,33 @@ int ensure_index_buffers(gpj_ctx* ctx, gpj_file* f, int num_levels) {
     if (num_levels < 1 || num_levels > GPJ_MAX_LEVELS)
         return fail(ctx, GPJ_ELIMIT, "Invalid number of levels: " + std::to_string(num_levels));
     if (!f->d_str) {
-        // one allocation: string index, key marks, levels, newlines, odd words
+        // one allocation: string index, key marks, levels, newlines, odd words.
+        // Large files take one for each part instead, of which the pool finds
+        // freed ones of the same size: with one of 1.6 GB, some loads of 2 GiB
+        // took 4 to 20 ms longer (one 460) than the 41 of the others
         const int64_t lines = std::min<int64_t>(f->n + 1, f->n / 256 + 1024);
-        rc = device_alloc(ctx, &f->d_str,
-                          static_cast<size_t>((2 + num_levels) * f->stride + lines + (f->words + 63) / 64),
-                          "cudaMalloc(index)");
-        if (rc) return rc;
-        f->d_marks = f->d_str + f->stride;
-        f->d_lvl = f->d_marks + f->stride;
-        f->lvl_cap = num_levels;
-        f->d_nl = reinterpret_cast<int64_t*>(f->d_lvl + num_levels * f->stride);
-        f->nl_cap = lines;
-        f->d_odd = reinterpret_cast<uint32_t*>(f->d_nl + lines);
-        f->lvl_inside = f->nl_inside = true;
+        const int64_t odd_words = (f->words + 63) / 64;
+        f->apart = f->n >= kApartBytes;
+        if (f->apart) {
+            rc = device_alloc(ctx, &f->d_marks, static_cast<size_t>(f->stride + odd_words), "cudaMalloc(key marks)");
+            if (!rc) rc = device_alloc(ctx, &f->d_str, static_cast<size_t>(f->stride), "cudaMalloc(string index)");
+            if (rc) {
+                device_free(ctx, f->d_marks);
+                return rc;
+            }
+            f->d_odd = reinterpret_cast<uint32_t*>(f->d_marks + f->stride);
+        } else {
+            rc = device_alloc(ctx, &f->d_str, static_cast<size_t>((2 + num_levels) * f->stride + lines + odd_words),
+                              "cudaMalloc(index)");
+            if (rc) return rc;
+            f->d_marks = f->d_str + f->stride;
+            f->d_lvl = f->d_marks + f->stride;
+            f->lvl_cap = num_levels;
+            f->d_nl = reinterpret_cast<int64_t*>(f->d_lvl + num_levels * f->stride);
+            f->nl_cap = lines;
+            f->d_odd = reinterpret_cast<uint32_t*>(f->d_nl + lines);
+            f->lvl_inside = f->nl_inside = true;
+        }
     }
     if (f->lvl_cap < num_levels) {
         free_levels(ctx, f);
@@ -1752,6 +1771,7 @@ void gpj_file_release(gpj_file* f) {
         free_levels(ctx, f);
         free_newlines(ctx, f);
         device_free(ctx, f->d_str);
+        if (f->apart) device_free(ctx, f->d_marks);
         device_free(ctx, f->d_ir);
         device_free(ctx, f->d_out);
     }
@@ -2114,8 +2134,7 @@ namespace {
 // Indexes the batch's files whose resident index is missing or too shallow:
 // one standalone index launch over all their tiles, one newline pass, one
 // status read-back.  Files the batch launch cannot index (not line-delimited,
-// a line longer than the look-ahead allows, more lines than estimated) are
-// indexed again alone.
+// more lines than estimated) are indexed again alone.
 int batch_index(gpj_ctx* ctx, std::vector<gpj_batch::FileRun>& files) {
     std::vector<gpj_file*> need;
     int levels = 1;
