@@ -31,14 +31,14 @@
 // summaries), and after their level changes (one shuffle scan).  The level
 // split is bit-parallel (split_half), so no lane waits for a denser word.
 //
-// Bound by integer operations: the ALU pipe is 84 % busy at 256 MiB of tweets
-// (128 us, DRAM bytes = input + index, 0.38 warp instructions per byte),
-// DRAM at a third of its rate.  The kernel this one replaced (30 KiB tiles
+// Bound by integer operations: the ALU pipe is 83 % busy at 256 MiB of tweets
+// (128 us, DRAM bytes = input + index, 0.41 warp instructions per byte),
+// DRAM at 43 % of its rate.  The kernel this one replaced (30 KiB tiles
 // with a 2 KiB look-ahead each, word state kept in shared memory between two
 // passes, the level split dealt over the warp by cuts) took 193 us there.
-// Index builds: 2 GiB of tweets 1558 -> 1102 us; 1 GiB with lines up to 1 MiB,
-// which went to the exact kernel before, 1287 -> 888 us; 256 MiB of it at 16
-// levels 900 -> 276 us; 256 MiB of 117-byte lines 269 -> 178 us.
+// Index builds: 2 GiB of tweets 1558 -> 1076 us; 1 GiB with lines up to 1 MiB,
+// which went to the exact kernel before, 1287 -> 833 us; 256 MiB of it at 16
+// levels 900 -> 262 us; 256 MiB of 117-byte lines 269 -> 166 us.
 #include <cstdint>
 
 #include "device_common.cuh"

@@ -87,13 +87,15 @@ int gpj_set_stream(gpj_ctx *ctx, void *stream);
  * 512x1024 for find_value, stages/CombinedIndex.java:28-56,
  * functions/QueryFunction.java:201-241).  Results do not depend on them.
  *  - long_line_bytes: find_value evaluates lines longer than this with a
- *    whole warp each instead of one thread (0 = the default, 65536; -1 = never);
+ *    whole warp each instead of one thread.  0 = the default, 65536: then
+ *    lines from 8 KiB on, and all lines of a file that has few (line, query)
+ *    pairs or long lines on average, get a warp.  -1 = never;
  *  - query_ctas_per_sm, index_ctas_per_sm: resident CTAs per SM of
  *    find_value and of the standalone index kernel (0 = the occupancy
  *    maximum; larger values are capped at it);
  *  - chunk_tiles: gpj_index_query_device and gpj_query_paths build the index
- *    and evaluate the queries chunk by chunk, chunks of this many 30 KiB
- *    tiles (a multiple of 1024), so that find_value reads each chunk's index
+ *    and evaluate the queries chunk by chunk, chunks of this many units
+ *    of 30 KiB (a multiple of 1024), so that find_value reads each chunk's index
  *    from L2 right after it is written (0, the default = one index pass over
  *    the whole file, then one find_value pass; on tweet-like NDJSON the
  *    whole-file passes are faster, since find_value needs more lines than a
