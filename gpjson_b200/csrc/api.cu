@@ -943,13 +943,14 @@ int ensure_index_buffers(gpj_ctx* ctx, gpj_file* f, int num_levels) {
         const int64_t odd_words = (f->words + 63) / 64;
         f->apart = f->n >= kApartBytes;
         if (f->apart) {
-            rc = device_alloc(ctx, &f->d_marks, static_cast<size_t>(f->stride + odd_words), "cudaMalloc(key marks)");
-            if (!rc) rc = device_alloc(ctx, &f->d_str, static_cast<size_t>(f->stride), "cudaMalloc(string index)");
+            rc = device_alloc(ctx, &f->d_str, static_cast<size_t>(f->stride), "cudaMalloc(string index)");
+            if (!rc) rc = device_alloc(ctx, &f->d_marks, static_cast<size_t>(f->stride), "cudaMalloc(key marks)");
+            if (!rc) rc = device_alloc(ctx, &f->d_odd, static_cast<size_t>(2 * odd_words), "cudaMalloc(odd words)");
             if (rc) {
+                device_free(ctx, f->d_str);
                 device_free(ctx, f->d_marks);
                 return rc;
             }
-            f->d_odd = reinterpret_cast<uint32_t*>(f->d_marks + f->stride);
         } else {
             rc = device_alloc(ctx, &f->d_str, static_cast<size_t>((2 + num_levels) * f->stride + lines + odd_words),
                               "cudaMalloc(index)");
@@ -1771,7 +1772,10 @@ void gpj_file_release(gpj_file* f) {
         free_levels(ctx, f);
         free_newlines(ctx, f);
         device_free(ctx, f->d_str);
-        if (f->apart) device_free(ctx, f->d_marks);
+        if (f->apart) {
+            device_free(ctx, f->d_marks);
+            device_free(ctx, f->d_odd);
+        }
         device_free(ctx, f->d_ir);
         device_free(ctx, f->d_out);
     }
