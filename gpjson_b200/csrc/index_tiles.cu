@@ -59,7 +59,8 @@ constexpr int kBefore = 16;  // bytes before the tile kept with it (escapes)
 
 // Tile states, three words per tile (tagged with the launch epoch in the top
 // 16 bits where other tiles poll them):
-//   [0] effect of a tile without '\n': q(1) | dd0 + 16384 (16) | ddt + 16384 (16)
+//   [0] effect of a tile without '\n': e(1) | q(1) | dd0 + 16384 (16) | ddt + 16384 (16);
+//       e: of a tile of backslashes alone, the escape state of its first byte
 //   [1] end state: s(1) | d + 2^46 (47)
 //   [2] start state, as [1] (read after the launch only)
 constexpr unsigned long long kPayload = (1ull << 48) - 1;
@@ -99,6 +100,11 @@ struct __align__(128) Shared {
     int32_t dd0[kWarps], ddt[kWarps];
     int32_t s0;
     int64_t d0;
+    // the launch's, for escape_before (arguments cost the kernel registers)
+    const unsigned long long* states;
+    unsigned long long* status;
+    uint32_t epoch;
+    uint32_t escape;  // escape state of the tile's first byte, where a backslash is before it
 };
 
 __device__ __forceinline__ uint8_t* tile_bytes(Shared& sh) { return sh.slot + 128; }
@@ -121,17 +127,70 @@ __device__ __forceinline__ void claim_tile(const IndexParams& p, Shared& sh, uin
     load_slot(F.file, start - lead, bytes + lead, tile_bytes(sh) - lead, &sh.full);
 }
 
-// Escape state of the byte at `w` bytes into the tile: parity of the run of
-// backslashes before it, in the slot and, where it fills the 16 bytes before
-// the tile too, on in device memory.
-__device__ __noinline__ uint32_t escape_before(const uint8_t* bytes, int w, const uint8_t* file, int64_t tile_start) {
+// Parity of the run of backslashes that ends the 16 bytes of v, -1 where they
+// are all backslashes.
+__device__ __forceinline__ int run_at_end(const uint4& v) {
+    const uint32_t w = ~eq_bytes(v.w, 0x5C5C5C5Cu) & 0x80808080u, z = ~eq_bytes(v.z, 0x5C5C5C5Cu) & 0x80808080u;
+    const uint32_t y = ~eq_bytes(v.y, 0x5C5C5C5Cu) & 0x80808080u, x = ~eq_bytes(v.x, 0x5C5C5C5Cu) & 0x80808080u;
+    const uint32_t d = w ? w : (z ? z : (y ? y : x));  // four more bytes do not change the parity
+    return d ? (clz32(d) >> 3) & 1 : -1;
+}
+
+// The answer of the first lane that has one, or -1.
+__device__ __forceinline__ int first_answer(int mine) {
+    const unsigned has = __ballot_sync(~0u, mine >= 0);
+    return has ? __shfl_sync(~0u, mine, __ffs(static_cast<int>(has)) - 1) : -1;
+}
+
+// Escape state of the byte at `w` (a multiple of 16) bytes into the tile of
+// buffer b: parity of the run of backslashes before it.  A whole warp calls
+// it, where the byte before is a backslash: 16 bytes a lane, back through the
+// slot and then the tile before in device memory (four loads in flight).  A
+// tile before that is backslashes throughout passes on the state of its own
+// first byte, which it publishes with its effect, so a run of any length costs
+// each of its tiles one such look and one wait: bound by that chain, 1.4 us a
+// tile (a build with one run of 33 MiB 2.9 ms, of 512 MiB 45 ms; of as many
+// other bytes 0.07 and 0.5 ms).  Each word for itself walking back to the
+// run's first byte costs the square of its length.
+__device__ __noinline__ uint32_t escape_before(Shared& sh, int b, int w) {
+    const int lane = threadIdx.x & 31;
+    const uint8_t* const bytes = tile_bytes(sh);
+    const int64_t tile_start = (sh.tile[b] - sh.desc[b].tile_begin) * kTile;
     const int floor = tile_start > 0 ? -kBefore : 0;
-    int k = w - 1;
-    while (k >= floor && bytes[k] == '\\') --k;
-    int64_t run = w - 1 - k;
-    if (k < floor)
-        for (int64_t g = tile_start + floor - 1; g >= 0 && file[g] == '\\'; --g) ++run;
-    return static_cast<uint32_t>(run & 1);
+    for (int at = w; at > floor; at -= 512) {
+        const int a = at - 16 * (lane + 1);
+        const int r = first_answer(a >= floor ? run_at_end(*reinterpret_cast<const uint4*>(bytes + a))
+                                              : (tile_start > 0 ? -1 : 0));
+        if (r >= 0) return static_cast<uint32_t>(r);
+    }
+    if (tile_start == 0) return 0;
+    const uint8_t* const tile_before = sh.desc[b].file + (tile_start - kTile);
+    for (int at = static_cast<int>(kTile) - kBefore; at > 0; at -= 4 * 512) {
+        int mine[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int a = at - 512 * c - 16 * (lane + 1);
+            mine[c] = a >= 0 ? run_at_end(*reinterpret_cast<const uint4*>(tile_before + a)) : -1;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int r = first_answer(mine[c]);
+            if (r >= 0) return static_cast<uint32_t>(r);
+        }
+    }
+    if (tile_start == kTile) return 0;  // the run begins with the file
+    const unsigned long long* const before = sh.states + 3 * (sh.tile[b] - 1);
+    for (unsigned polls = 1;; ++polls) {
+        const unsigned long long g = __shfl_sync(~0u, ld_state(before), 0);
+        if (has_tag(g, sh.epoch)) return static_cast<uint32_t>((g >> 33) & 1);
+        const bool expired =
+            polls > kMaxPolls || ((polls & 1023u) == 0 && __any_sync(~0u, (ld_acquire(sh.status + 1) & kFatalErrors) != 0));
+        if (expired) {
+            if (lane == 0) atomicOr(sh.status + 1, kErrLookbackTimeout);
+            return 0;  // the host reports the error; outputs are not valid
+        }
+        __nanosleep(64);
+    }
 }
 
 // State before tile t of a file whose first tile is t0 (one warp): the tiles
@@ -224,6 +283,9 @@ __global__ void __launch_bounds__(kThreads, LV <= 8 ? 6 : 5) tile_index_kernel(I
     const unsigned lt_mask = (1u << lane) - 1;
     uint8_t* const bytes = tile_bytes(sh);
     if (tid == 0) {
+        sh.states = p.tile_state;
+        sh.status = p.status;
+        sh.epoch = p.epoch;
         mbar_init(&sh.full, 1);
         fence_mbar_init();
         claim_tile(p, sh, 0);
@@ -272,17 +334,20 @@ __global__ void __launch_bounds__(kThreads, LV <= 8 ? 6 : 5) tile_index_kernel(I
             // before it; a warp without backslashes can only have its first
             // byte escaped
             ballot_b = __ballot_sync(~0u, bs != 0);
-            uint32_t cin = 0;
-            if (lane == 0 && (tid > 0 || tile_start > 0) && bytes[64 * tid - 1] == '\\')
-                cin = escape_before(bytes, 64 * tid, F.file, tile_start);
+            const int first = 64 * 32 * warp;
+            uint32_t cin = 0;  // of the warp's first byte
+            if ((warp > 0 || tile_start > 0) && bytes[first - 1] == '\\') {
+                cin = escape_before(sh, b, first);
+                if (tid == 0) sh.escape = cin;
+            }
             if (ballot_b) {
+                // (a word of backslashes passes on what it was given)
                 const unsigned runs = __ballot_sync(~0u, trailing_run_odd(bs));
-                if (lane > 0) cin = (runs >> (lane - 1)) & 1u;
-                const unsigned full = __ballot_sync(~0u, bs == ~0ull);
-                if (lane > 0 && ((full >> (lane - 1)) & 1u)) cin = escape_before(bytes, 64 * tid, F.file, tile_start);
+                const unsigned stops = ~__ballot_sync(~0u, bs == ~0ull) & lt_mask;
+                if (stops) cin = (runs >> (31 - clz32(stops))) & 1u;
                 quote &= ~escaped_bytes(bs, cin);
             } else {
-                quote &= ~static_cast<uint64_t>(cin);
+                quote &= ~static_cast<uint64_t>(lane ? 0u : cin);
             }
             p0 = prefix_xor_halves(quote);
         }
@@ -316,9 +381,17 @@ __global__ void __launch_bounds__(kThreads, LV <= 8 ? 6 : 5) tile_index_kernel(I
                     sh.dd0[warp] = dd0;
                     sh.ddt[warp] = ddt;
                 }
-                __syncthreads();
+                // a tile of backslashes alone (its words still lie in the slot)
+                bool passes = ballot_b == ~0u && !tail;
+                if (passes) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        passes = passes && run_at_end(*reinterpret_cast<const uint4*>(bytes + 64 * tid + 16 * i)) < 0;
+                }
+                const bool all_pass = __syncthreads_and(passes);
                 if (warp == 0) {
                     if (lane == 0) {
+                        const unsigned long long escape = all_pass && bytes[-1] == '\\' ? sh.escape : 0;
                         int e0 = 0, et = 0;
 #pragma unroll
                         for (int w = 0; w < kWarps; w++) {
@@ -326,7 +399,8 @@ __global__ void __launch_bounds__(kThreads, LV <= 8 ? 6 : 5) tile_index_kernel(I
                             et += sh.ddt[w];
                         }
                         st_state(p.tile_state + 3 * t,
-                                 tagged(p.epoch, (static_cast<unsigned long long>(popc64(warps_q) & 1) << 32) |
+                                 tagged(p.epoch, (escape << 33) |
+                                                     (static_cast<unsigned long long>(popc64(warps_q) & 1) << 32) |
                                                      (static_cast<unsigned long long>(e0 + 16384) << 16) |
                                                      static_cast<unsigned long long>(et + 16384)));
                     }
