@@ -883,7 +883,7 @@ int warp_grid(const gpj_ctx* ctx, int64_t items, bool listed) {
 // [d_range[0], d_range[1]) of a file whose index is still being built
 // (`last`: they include the file's last line).
 int launch_query(gpj_ctx* ctx, gpj_file* f, int nq, int slots, int64_t* d_out, int64_t out_lines,
-                 const int64_t* d_range = nullptr, bool last = false) {
+                 const int64_t* d_range = nullptr, bool last = false, int64_t hi = INT64_MAX) {
     cudaStream_t stream = ctx->stream;
     gpj::QueryParams p{};
     p.file = f->d_data;
@@ -902,6 +902,8 @@ int launch_query(gpj_ctx* ctx, gpj_file* f, int nq, int slots, int64_t* d_out, i
     p.range = d_range;
     p.last = last ? 1 : 0;
     p.newline_cap = f->nl_cap;
+    p.hi = std::min(hi, f->n);
+    p.status = ctx->d_status;
     p.marks = f->marks_valid ? f->d_marks : nullptr;
     p.odd = f->marks_valid ? f->d_odd : nullptr;
     p.depth = f->ir_depth;
@@ -1020,14 +1022,14 @@ struct ChunkQueries {
 };
 
 // Copies n host bytes into f->d_owned in chunks on the copy stream and
-// indexes chunk k with the line-parallel kernel as soon as chunk k + 1 has
-// landed (a line starting in chunk k ends in chunk k + 1 unless it is longer
-// than a chunk), so the copy and the index build overlap.  With `cq`, the
-// newline index of chunk k follows at once, and then find_value on the
-// lines it completes, so the queries overlap the copy too (*queries_done
-// tells whether they all ran that way).  Inputs the line kernel cannot
-// index this way (not NDJSON, or a line longer than a chunk) are indexed
-// again from the complete copy by run_index.
+// indexes chunk k with the standalone kernel as soon as chunk k + 1 has
+// landed, so the copy and the index build overlap.  With `cq`, the newline
+// index of chunk k follows at once, and then find_value on the lines it
+// completes, so the queries overlap the copy too (*queries_done tells whether
+// they all ran that way).  find_value reads no further than chunk k + 1: only
+// a whitespace skip can want to, from a line into blank ones after it, and
+// then the queries count as not done.  Inputs the standalone kernel cannot
+// index (not NDJSON) are indexed again from the complete copy by run_index.
 //
 // host == nullptr: the input is already in f->d_data; chunks of
 // `chunk_units` x 30 KiB are indexed and queried in turn (index kernel, newline
@@ -1112,7 +1114,8 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
             GPJ_CUDA(ctx, gpj::launch_newline_index_range(p, ts.offsets, t0, t1, d_lines + k + 1, static_cast<int>(grid),
                                                           ctx->stream));
             ctx->launches += 2;
-            return launch_query(ctx, f, cq->nq, cq->slots, cq->d_out, cq->out_lines, d_lines + k, k == nchunks - 1);
+            return launch_query(ctx, f, cq->nq, cq->slots, cq->d_out, cq->out_lines, d_lines + k, k == nchunks - 1,
+                                resident ? n : (k + 2) * chunk_bytes);
         };
         for (int64_t k = 0; k < nchunks && !rc; k++) {
             if (resident) {
@@ -1154,7 +1157,7 @@ int load_and_index(gpj_ctx* ctx, gpj_file* f, const uint8_t* host, int num_level
         } else if ((rc = status_error(ctx, errs))) {
             f->marks_valid = false;
             return rc;
-        } else if (cq && lines <= f->nl_cap && lines <= cq->out_lines && queries_done) {
+        } else if (cq && !(errs & gpj::kErrDeferred) && lines <= f->nl_cap && lines <= cq->out_lines && queries_done) {
             *queries_done = true;
         }
     }

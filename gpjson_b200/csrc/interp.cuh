@@ -700,7 +700,7 @@ GPJ_HD int run_line(const LineView& v, int64_t line_start, int64_t line_end, Ir 
             v.file + base, n, hi, skip_end, v.string_index + w, v.levels + w, v.level_size,
             v.colon ? v.colon + w : nullptr, v.odd, static_cast<int32_t>(line_start - base),
             static_cast<int32_t>(line_end - base), code_of(ir), res, base, lv, stored);
-        if (r != kLineDeferred || !clamped || v.hi < v.n) {
+        if (r != kLineDeferred || !clamped) {
             for (int64_t k = 2 * static_cast<int64_t>(stored); k < res_len; k++) Scan::store(res, k, -1);
             return r;
         }

@@ -25,6 +25,7 @@
 // (query_program.h).
 #include <cstdint>
 
+#include "device_common.cuh"
 #include "interp.cuh"
 #include "query_items.cuh"
 #include "query_kernel.h"
@@ -202,7 +203,7 @@ __device__ __forceinline__ int64_t handed_over(const LongLines& L) {
 template <int D, int K>
 __global__ void __launch_bounds__(kQueryThreads, kQueryMinCtas<D>) find_value_kernel(QueryParams p) {
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    const LineView view{p.file, p.n, p.string_index, p.leveled, p.level_size, p.n, p.marks, p.odd};
+    const LineView view{p.file, p.n, p.string_index, p.leveled, p.level_size, p.hi, p.marks, p.odd};
     const int64_t per_line = 2 * static_cast<int64_t>(p.slots);
     // lines [first, first + lines); the file's last line ends at p.n
     int64_t first = 0, lines = p.num_lines, file_lines = p.num_lines;
@@ -226,10 +227,10 @@ __global__ void __launch_bounds__(kQueryThreads, kQueryMinCtas<D>) find_value_ke
         const ProgramCode ir{p.programs + p.offsets[q]};
         // writes every slot once, unless a whitespace skip runs far past the
         // line (then a warp evaluates it again)
-        if (run_line<D, SeqScanOf<K>>(view, start, end, ir, res, per_line, kRelLimit,
-                                      p.long_lines.items ? p.long_lines.bytes : -1) == kLineLong &&
-            !hand_over(p.long_lines, i, 0, q))
-            run_line_wide(view, start, end, ir, res, per_line);
+        int r = run_line<D, SeqScanOf<K>>(view, start, end, ir, res, per_line, kRelLimit,
+                                          p.long_lines.items ? p.long_lines.bytes : -1);
+        if (r == kLineLong && !hand_over(p.long_lines, i, 0, q)) r = run_line_wide(view, start, end, ir, res, per_line);
+        if (r == kLineDeferred) atomicOr(p.status + 1, kErrDeferred);
     }
 }
 
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(kWarpThreads, kWarpMinCtas<D>) find_value_warp
     const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     const int64_t own = p.by_warp ? p.num_lines * p.num_queries : 0;
     const int64_t count = own + handed_over(p.long_lines);
-    const LineView view{p.file, p.n, p.string_index, p.leveled, p.level_size, p.n, p.marks, p.odd};
+    const LineView view{p.file, p.n, p.string_index, p.leveled, p.level_size, p.hi, p.marks, p.odd};
     const int64_t per_line = 2 * static_cast<int64_t>(p.slots);
     const int64_t file_lines = p.range ? (p.last ? p.range[1] : INT64_MAX) : p.num_lines;
     for (int64_t k = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; k < count; k += warps) {
@@ -252,8 +253,10 @@ __global__ void __launch_bounds__(kWarpThreads, kWarpMinCtas<D>) find_value_warp
         const int64_t start = p.newlines[it.line];
         const int64_t end = it.line + 1 >= file_lines ? p.n : p.newlines[it.line + 1];
         int64_t* res = p.out + (static_cast<int64_t>(it.query) * p.out_lines + it.line) * per_line;
-        run_line<D, WarpScan>(view, start, end, ProgramCode{p.programs + p.offsets[it.query]}, res,
-                                    per_line);
+        if (run_line<D, WarpScan>(view, start, end, ProgramCode{p.programs + p.offsets[it.query]}, res, per_line) ==
+                kLineDeferred &&
+            (threadIdx.x & 31) == 0)
+            atomicOr(p.status + 1, kErrDeferred);
     }
 }
 

@@ -68,6 +68,11 @@ struct QueryParams {
     const int64_t* range;
     int last;
     int64_t newline_cap;
+    // Bytes at or after `hi` are not read (n: all may be; else, with `range`,
+    // they are still on their way to the device): a query whose whitespace
+    // skip gets there sets kErrDeferred in status[1], its results are not valid.
+    int64_t hi;
+    unsigned long long* status;
     // Optional (both or none), IndexParams::marks and odd: key searches jump
     // between the ':' of keys of the right length, index searches between the
     // other structural bytes.
