@@ -519,11 +519,16 @@ int end_phase(gpj_ctx* ctx, const char* name, double host_start) {
 int ensure_tile_state(gpj_ctx* ctx, int64_t ntiles) {
     const int64_t words = 3 * ntiles;
     if (words > ctx->tile_state_words) {
-        device_free(ctx, ctx->d_tile_state);
+        // Not from the pool: what stays there among a file's buffers keeps the
+        // next file's from the place of the last one's, and the pool remaps
+        // memory for them at every load (2 GiB with little to spare: 41.3 ms
+        // a load, now and then 50 to 1000, instead of 40.7)
+        const int64_t cap = std::max<int64_t>({words, 3 * 4096, ctx->tile_state_words * 3 / 2});
+        GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        if (ctx->d_tile_state) cudaFree(ctx->d_tile_state);
+        ctx->d_tile_state = nullptr;
         ctx->tile_state_words = 0;
-        const int64_t cap = std::max<int64_t>(words, 3 * 4096);
-        int rc = device_alloc(ctx, &ctx->d_tile_state, static_cast<size_t>(cap), "cudaMalloc(tile state)");
-        if (rc) return rc;
+        GPJ_CUDA(ctx, cudaMalloc(&ctx->d_tile_state, static_cast<size_t>(cap) * 8));
         GPJ_CUDA(ctx, cudaMemsetAsync(ctx->d_tile_state, 0, cap * 8, ctx->stream));
         ctx->tile_state_words = cap;
         ctx->epoch = 0;
@@ -1420,9 +1425,9 @@ void gpj_destroy(gpj_ctx* ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->own_stream) {
         ctx->stream = ctx->own_stream;
-        device_free(ctx, ctx->d_tile_state);
         cudaStreamSynchronize(ctx->own_stream);
     }
+    if (ctx->d_tile_state) cudaFree(ctx->d_tile_state);
     if (ctx->d_long) cudaFree(ctx->d_long);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->copy_stream) {
