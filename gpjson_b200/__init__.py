@@ -607,11 +607,16 @@ class GPJSON:
                    index_ctas_per_sm: int | None = None, chunk_tiles: int | None = None) -> None:
         """gpj_set_tuning: changes the given launch shapes (results do not
         depend on them)."""
-        cur = self.tuning()
-        t = _lib.Tuning(cur["long_line_bytes"] if long_line_bytes is None else long_line_bytes,
-                        cur["query_ctas_per_sm"] if query_ctas_per_sm is None else query_ctas_per_sm,
-                        cur["index_ctas_per_sm"] if index_ctas_per_sm is None else index_ctas_per_sm,
-                        cur["chunk_tiles"] if chunk_tiles is None else chunk_tiles, 0)
+        t = _lib.Tuning()
+        self._native.check(self._native.lib.gpj_get_tuning(self._native.h, byref(t)))
+        if long_line_bytes is not None:
+            t.long_line_bytes, t.reserved = long_line_bytes, 0
+        if query_ctas_per_sm is not None:
+            t.query_ctas_per_sm = query_ctas_per_sm
+        if index_ctas_per_sm is not None:
+            t.index_ctas_per_sm = index_ctas_per_sm
+        if chunk_tiles is not None:
+            t.chunk_tiles = chunk_tiles
         self._native.check(self._native.lib.gpj_set_tuning(self._native.h, byref(t)))
 
     def set_stream(self, stream_handle: int | None) -> None:

@@ -81,6 +81,7 @@ static gpj_tuning default_tuning() {
     t.query_ctas_per_sm = 0;
     t.index_ctas_per_sm = 0;
     t.chunk_tiles = 0;
+    t.reserved = 1;  // (choose_warps)
     return t;
 }
 
@@ -865,13 +866,15 @@ int query_occupancy(const gpj_ctx* ctx, int depth) {
     return want > 0 && want < occ ? want : occ;
 }
 
-// The hand-over of long lines to a warp each, or none (tuning.long_line_bytes
-// < 0).  The tuning's default stands for the library's choice.
+// Whether the library chooses the lines that get a warp (else
+// tuning.long_line_bytes alone does).
+bool choose_warps(const gpj_ctx* ctx) { return ctx->tuning.reserved != 0; }
+
+// The hand-over of long lines to a warp each, or none (tuning.long_line_bytes < 0).
 gpj::LongLines long_lines(const gpj_ctx* ctx) {
     const int64_t set = ctx->tuning.long_line_bytes;
     if (set < 0 || !ctx->d_long) return gpj::LongLines{nullptr, nullptr, 0, 0};
-    return gpj::LongLines{ctx->d_long, ctx->d_long_count, kLongItems,
-                          set == default_tuning().long_line_bytes ? kLongLineBytes : set};
+    return gpj::LongLines{ctx->d_long, ctx->d_long_count, kLongItems, choose_warps(ctx) ? kLongLineBytes : set};
 }
 
 // Grid of a warp-per-line launch over `items` pairs (and, `listed`, an
@@ -913,7 +916,7 @@ int launch_query(gpj_ctx* ctx, gpj_file* f, int nq, int slots, int64_t* d_out, i
     p.odd = f->marks_valid ? f->d_odd : nullptr;
     p.depth = f->ir_depth;
     // (a chunk's lines are not counted yet)
-    p.by_warp = !d_range && ctx->tuning.long_line_bytes >= 0 &&
+    p.by_warp = !d_range && choose_warps(ctx) &&
                 gpj::query_by_warp(f->num_lines, f->n, nq, kFewPairs);
     p.short_lines = !d_range && f->n / gpj::kShortLineBytes < f->num_lines;
     if (!p.by_warp) p.long_lines = long_lines(ctx);
@@ -1460,8 +1463,14 @@ int gpj_set_tuning(gpj_ctx* ctx, const gpj_tuning* tuning) {
         return fail(ctx, GPJ_EINVAL, "CTAs per SM must be >= 0");
     if (tuning->chunk_tiles < 0 || tuning->chunk_tiles % 1024 != 0)
         return fail(ctx, GPJ_EINVAL, "chunk_tiles must be a multiple of 1024 (0 = whole-file passes)");
+    const gpj_tuning def = default_tuning();
     ctx->tuning = *tuning;
-    if (ctx->tuning.long_line_bytes == 0) ctx->tuning.long_line_bytes = default_tuning().long_line_bytes;
+    if (tuning->long_line_bytes == 0 || (tuning->long_line_bytes == def.long_line_bytes && tuning->reserved == def.reserved)) {
+        ctx->tuning.long_line_bytes = def.long_line_bytes;
+        ctx->tuning.reserved = def.reserved;
+    } else {
+        ctx->tuning.reserved = 0;
+    }
     return GPJ_OK;
 }
 
@@ -2357,7 +2366,7 @@ int gpj_batch_run(gpj_batch* b) {
     std::vector<size_t> order;
     for (size_t i = 0; i < b->files.size(); i++) {
         auto& fr = b->files[i];
-        fr.by_warp = ctx->tuning.long_line_bytes >= 0 &&
+        fr.by_warp = choose_warps(ctx) &&
                      (pairs <= kFewBatchPairs ||
                       gpj::query_by_warp(fr.lines, fr.file->n, static_cast<int>(fr.queries.size()), 0));
         if (!fr.by_warp) order.push_back(i);
@@ -2402,7 +2411,8 @@ int gpj_batch_run(gpj_batch* b) {
                     (gr.warp_items > 0 || (gr.items > 0 && long_lines(ctx).items) ? 1 : 0);
     // what the query phase reads: replay its graph when nothing of it changed
     std::vector<uint64_t> sig{static_cast<uint64_t>(reinterpret_cast<uintptr_t>(ctx->stream)),
-                              static_cast<uint64_t>(ctx->tuning.long_line_bytes)};
+                              static_cast<uint64_t>(ctx->tuning.long_line_bytes),
+                              static_cast<uint64_t>(choose_warps(ctx))};
     for (const BatchGroup& gr : groups) sig.push_back(static_cast<uint64_t>(query_occupancy(ctx, gr.depth)));
     for (auto& fr : b->files) {
         gpj_file* f = fr.file;

@@ -87,9 +87,11 @@ int gpj_set_stream(gpj_ctx *ctx, void *stream);
  * 512x1024 for find_value, stages/CombinedIndex.java:28-56,
  * functions/QueryFunction.java:201-241).  Results do not depend on them.
  *  - long_line_bytes: find_value evaluates lines longer than this with a
- *    whole warp each instead of one thread.  0 = the default, 65536: then
- *    lines from 8 KiB on, and all lines of a file that has few (line, query)
- *    pairs or long lines on average, get a warp.  -1 = never;
+ *    whole warp each instead of one thread, and only these; -1 = never.  0,
+ *    the default, leaves it to the library: lines from 8 KiB on, and all lines
+ *    of a file that has few (line, query) pairs or long lines on average, get
+ *    a warp.  gpj_get_tuning then gives 65536 and reserved 1, which
+ *    gpj_set_tuning takes back for the same;
  *  - query_ctas_per_sm, index_ctas_per_sm: resident CTAs per SM of
  *    find_value and of the standalone index kernel (0 = the occupancy
  *    maximum; larger values are capped at it);
@@ -100,7 +102,7 @@ int gpj_set_stream(gpj_ctx *ctx, void *stream);
  *    the whole file, then one find_value pass; on tweet-like NDJSON the
  *    whole-file passes are faster, since find_value needs more lines than a
  *    chunk holds to hide its load latency);
- *  - reserved: 0.
+ *  - reserved: 0 (or as gpj_get_tuning gave it).
  * gpjson_b200.tune (Python) measures and persists them per device. */
 typedef struct gpj_tuning {
     int64_t long_line_bytes;
