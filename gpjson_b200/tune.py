@@ -28,14 +28,20 @@ from pathlib import Path
 KNOBS = ("index_ctas_per_sm", "query_ctas_per_sm", "long_line_bytes", "chunk_tiles")
 ENV = {"long_line_bytes": "GPJSON_LONG_LINE_BYTES", "query_ctas_per_sm": "GPJSON_QUERY_CTAS_PER_SM",
        "index_ctas_per_sm": "GPJSON_INDEX_CTAS_PER_SM", "chunk_tiles": "GPJSON_CHUNK_TILES"}
-# candidates per knob (0 = the library's default: the occupancy maximum, 64 KiB,
-# or whole-file passes)
+# candidates per knob (0 = the library's default: the occupancy maximum, its
+# choice of the lines that get a warp, or whole-file passes).  No line a warp
+# (-1) is none: it saves one short launch on a sample without long lines and
+# takes several times as long on files with them (lines up to 1 MiB 870 us
+# instead of 207, a request of 610 pairs 60 instead of 15).
 CANDIDATES = {
     "index_ctas_per_sm": [0, 2, 3, 4],
     "query_ctas_per_sm": [0, 2, 4, 6],
-    "long_line_bytes": [0, 16384, 262144, -1],
+    "long_line_bytes": [0, 16384, 262144],
     "chunk_tiles": [0, 2048],
 }
+# Line length from which the library's own choice gives a line a warp: a
+# sample without such lines says nothing about the others.
+LONG_LINE_BYTES = 8192
 
 
 def search(measure: Callable[[dict], float], start: dict | None = None,
@@ -113,11 +119,22 @@ def _device_key_of(device: int) -> str:
 
 def apply(gpjson, device: int = 0) -> dict:
     """Applies the stored / environment setting to a GPJSON context; returns
-    what was applied."""
+    what was applied.  A stored long_line_bytes of -1 (a candidate once) is
+    left to the library, unless the environment says so."""
     setting = load(_device_key_of(device))
+    if setting.get("long_line_bytes") == -1 and not os.environ.get(ENV["long_line_bytes"], "").strip():
+        setting["long_line_bytes"] = 0
     if setting:
         gpjson.set_tuning(**{k: int(v) for k, v in setting.items() if k in KNOBS})
     return setting
+
+
+def _candidates(newlines, size: int) -> dict[str, list[int]]:
+    """CANDIDATES for a sample of `size` bytes with that newline index."""
+    import numpy as np
+
+    longest = int(np.diff(np.append(newlines, size)).max())
+    return dict(CANDIDATES, long_line_bytes=CANDIDATES["long_line_bytes"] if longest > LONG_LINE_BYTES else [0])
 
 
 def tune(gpjson, data, queries: list[str], levels: int, device: int = 0, repeats: int = 3, persist: bool = True,
@@ -139,6 +156,7 @@ def tune(gpjson, data, queries: list[str], levels: int, device: int = 0, repeats
     f.build_index(levels)
     slots = max(c.num_results for c in compiled)
     out = torch.empty((len(compiled), f.num_lines, slots, 2), dtype=torch.int64, device=dev.device)
+    candidates = _candidates(f.newline_index(), dev.numel())
 
     def measure(setting: dict) -> float:
         gpjson.set_tuning(**setting)
@@ -155,7 +173,7 @@ def tune(gpjson, data, queries: list[str], levels: int, device: int = 0, repeats
                    if k in ("build_index", "find_value", "index_and_query"))
 
     try:
-        best, seen = search(measure)
+        best, seen = search(measure, candidates=candidates)
     finally:
         f.release()
     gpjson.set_tuning(**best)
