@@ -29,6 +29,7 @@
 #include "jsonpath.h"
 #include "query_kernel.h"
 #include "query_program.h"
+#include "value_blocks.h"
 #include "values.h"
 
 namespace {
@@ -223,101 +224,16 @@ struct gpj_result {
     }
 };
 
-// Host memory of gathered values: page-locked (copied to at full speed, no
-// page faults) up to kMost in all, free blocks kept for later values of the
-// process until its last context is destroyed.  Larger ones are pageable.
-class ValueBlocks {
-  public:
-    static constexpr size_t kMost = size_t(64) << 20;
-
-    uint8_t* take(size_t size, size_t* cap, bool* pinned) {
-        bool grow = false;  // sizes vary: one that serves the next as well
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            size_t best = free_.size();
-            for (size_t i = 0; i < free_.size(); i++)
-                if (free_[i].second >= size && (best == free_.size() || free_[i].second < free_[best].second)) best = i;
-            if (best < free_.size()) {
-                const auto b = free_[best];
-                free_.erase(free_.begin() + best);
-                *cap = b.second;
-                *pinned = true;
-                return b.first;
-            }
-            grow = !free_.empty();
-        }
-        const size_t want = (size + (grow ? size / 4 : 0) + 0xFFFF) & ~size_t(0xFFFF);
+struct LockedPages {
+    static void* lock(size_t size) {
         void* p = nullptr;
-        *pinned = false;
-        if (reserve(want)) {
-            if (cudaMallocHost(&p, want) == cudaSuccess) {
-                *cap = want;
-                *pinned = true;
-                return static_cast<uint8_t*>(p);
-            }
-            cudaGetLastError();
-            unreserve(want);
-        }
-        *cap = size;
-        p = std::malloc(size);
-        if (p) std::memset(p, 0, size);  // a copy that faults in its own pages is slower
-        return static_cast<uint8_t*>(p);
+        if (cudaMallocHost(&p, size) == cudaSuccess) return p;
+        cudaGetLastError();
+        return nullptr;
     }
-
-    void give(uint8_t* p, size_t cap, bool pinned) {
-        if (!p) return;
-        if (!pinned) {
-            std::free(p);
-            return;
-        }
-        std::lock_guard<std::mutex> g(mu_);
-        try {
-            if (contexts_ > 0) {
-                free_.emplace_back(p, cap);
-                return;
-            }
-        } catch (const std::exception&) {
-            // no room to note it
-        }
-        total_ -= cap;
-        cudaFreeHost(p);
-    }
-
-    void context_created() {
-        std::lock_guard<std::mutex> g(mu_);
-        ++contexts_;
-    }
-    void context_destroyed() {
-        std::lock_guard<std::mutex> g(mu_);
-        if (--contexts_ == 0) drop_free();
-    }
-
-  private:
-    // Room for `size` more page-locked bytes, if need be in place of the free blocks.
-    bool reserve(size_t size) {
-        std::lock_guard<std::mutex> g(mu_);
-        if (total_ + size > kMost) drop_free();
-        if (total_ + size > kMost) return false;
-        total_ += size;
-        return true;
-    }
-    void unreserve(size_t size) {
-        std::lock_guard<std::mutex> g(mu_);
-        total_ -= size;
-    }
-    void drop_free() {
-        for (auto& b : free_) {
-            total_ -= b.second;
-            cudaFreeHost(b.first);
-        }
-        free_.clear();
-    }
-
-    std::mutex mu_;
-    std::vector<std::pair<uint8_t*, size_t>> free_;
-    size_t total_ = 0;  // page-locked bytes, in use or free
-    int contexts_ = 0;
+    static void unlock(void* p) { cudaFreeHost(p); }
 };
+using ValueBlocks = gpj::ValueBlocks<LockedPages>;
 
 // Never destroyed, so that values released during process exit find it.
 static ValueBlocks& value_blocks() {
