@@ -26,6 +26,7 @@
 #include "device_common.cuh"
 #include "host_io.h"
 #include "index_kernel.h"
+#include "index_layout.h"
 #include "jsonpath.h"
 #include "query_kernel.h"
 #include "query_program.h"
@@ -66,8 +67,9 @@ static constexpr int64_t kFewBatchPairs = 4096;
 // 1620 when the kernel writes the results to the host's memory itself.
 static constexpr size_t kGroupOut = size_t(8) << 17;
 
-// Inputs from this size on have their index in several allocations: an
-// allocation takes 2 us, a pass over them 100 and more.
+// Inputs from this size on have their index in several allocations, each
+// given back when it is replaced (an allocation takes 2 us, a pass over them
+// 100 and more).
 static constexpr int64_t kApartBytes = int64_t(128) << 20;
 
 // gpj_ctx::d_status and what follows it.
@@ -716,7 +718,7 @@ int make_file(gpj_ctx* ctx, int64_t n, gpj_file** out) {
     f->ctx = ctx;
     f->n = n;
     f->words = (n + 63) / 64;
-    f->stride = (f->words + 15) / 16 * 16;
+    f->stride = gpj::bitmap_words(n);
     *out = f;
     return GPJ_OK;
 }
@@ -862,11 +864,10 @@ int ensure_index_buffers(gpj_ctx* ctx, gpj_file* f, int num_levels) {
         return fail(ctx, GPJ_ELIMIT, "Invalid number of levels: " + std::to_string(num_levels));
     if (!f->d_str) {
         // one allocation: string index, key marks, levels, newlines, odd words.
-        // Large files take one for each part instead, of which the pool finds
-        // freed ones of the same size: with one of 1.6 GB, some loads of 2 GiB
-        // took 4 to 20 ms longer (one 460) than the 41 of the others
-        const int64_t lines = std::min<int64_t>(f->n + 1, f->n / 256 + 1024);
-        const int64_t odd_words = (f->words + 63) / 64;
+        // Large files take one for each part instead, so that an index with
+        // more levels later gives the first ones' memory back
+        const int64_t lines = gpj::first_lines(f->n, num_levels);
+        const int64_t odd_words = gpj::odd_words(f->n);
         f->apart = f->n >= kApartBytes;
         if (f->apart) {
             rc = device_alloc(ctx, &f->d_str, static_cast<size_t>(f->stride), "cudaMalloc(string index)");
@@ -878,8 +879,7 @@ int ensure_index_buffers(gpj_ctx* ctx, gpj_file* f, int num_levels) {
                 return rc;
             }
         } else {
-            rc = device_alloc(ctx, &f->d_str, static_cast<size_t>((2 + num_levels) * f->stride + lines + odd_words),
-                              "cudaMalloc(index)");
+            rc = device_alloc(ctx, &f->d_str, static_cast<size_t>(gpj::index_words(f->n, num_levels)), "cudaMalloc(index)");
             if (rc) return rc;
             f->d_marks = f->d_str + f->stride;
             f->d_lvl = f->d_marks + f->stride;
@@ -896,7 +896,7 @@ int ensure_index_buffers(gpj_ctx* ctx, gpj_file* f, int num_levels) {
         if (rc) return rc;
         f->lvl_cap = num_levels;
     }
-    if (!f->d_nl) return resize_newlines(ctx, f, std::min<int64_t>(f->n + 1, f->n / 256 + 1024));
+    if (!f->d_nl) return resize_newlines(ctx, f, gpj::first_lines(f->n, num_levels));
     return GPJ_OK;
 }
 

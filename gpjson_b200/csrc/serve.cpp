@@ -46,8 +46,9 @@ int64_t now_ns(std::chrono::steady_clock::time_point t0) {
     return std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now() - t0).count();
 }
 
-// Device bytes a corpus holds while resident: input, string index, ':'
-// bitmap, leveled bitmaps and the first newline-index allocation.
+// Device bytes a corpus holds while resident: input, string index, key marks,
+// leveled bitmaps and the first newline-index allocation (with the odd words
+// in its place: index_layout.h).
 int64_t resident_bytes(int64_t n, int levels) {
     const int64_t words = (n + 63) / 64;
     return n + 8 * words * (2 + levels) + 8 * (n / 256 + 1024);
