@@ -891,6 +891,7 @@ int ensure_index_buffers(gpj_ctx* ctx, gpj_file* f, int num_levels) {
         }
     }
     if (f->lvl_cap < num_levels) {
+        f->indexed = false;  // its bitmaps go, whether or not larger ones come
         free_levels(ctx, f);
         rc = device_alloc(ctx, &f->d_lvl, static_cast<size_t>(f->stride) * num_levels, "cudaMalloc(leveled bitmaps)");
         if (rc) return rc;
