@@ -309,7 +309,7 @@ struct gpj_batch {
     PinnedResults* cur = nullptr;
     bool ran = false;
     // The query phase of the last run as a CUDA graph (find_value over every
-    // item, the the copy of the results), replayed by the
+    // item, the copy of the results), replayed by the
     // next run when neither the requests nor the files' indexes nor the
     // launch shapes changed and no result of the last run is still held.
     struct Replay {
@@ -584,9 +584,9 @@ int finish_tiles(gpj_ctx* ctx, const gpj::IndexParams& p, const TileScratch& ts)
     return read_status(ctx);
 }
 
-// Builds the index with the line-parallel kernel (evaluating `fq` in the
-// same pass when given), and again with the exact kernel when the input is
-// not well-formed NDJSON.  *lines receives the line count; *queries_done
+// Builds the index with the standalone kernel (with the line-parallel kernel,
+// evaluating `fq` in the same pass, when given), and again with the exact
+// kernel when the input is not well-formed NDJSON.  *lines receives the line count; *queries_done
 // tells whether every line's query results were written.
 // `level_stride`: words from one level's bitmap to the next.
 // d_marks and d_odd (optional) receive the key marks when the standalone
@@ -2127,7 +2127,7 @@ int batch_index(gpj_ctx* ctx, std::vector<gpj_batch::FileRun>& files) {
                 gpj_file* f = batched[i];
                 const int64_t ntiles = (f->n + gpj::kStandaloneTileBytes - 1) / gpj::kStandaloneTileBytes;
                 tf.push_back(gpj::TileFile{f->d_data, f->n, f->n, f->d_str, f->d_lvl, f->stride, bits + word,
-                                           status + 2 * i, tile, nullptr, f->d_marks, f->d_odd});
+                                           status + 2 * i, tile, f->d_marks, f->d_odd});
                 lf.push_back(gpj::LineFile{bits + word, f->words, f->d_nl, f->nl_cap, status + 2 * i, tile, ntiles});
                 tile += ntiles;
                 word += f->words;

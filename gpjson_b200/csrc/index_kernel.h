@@ -1,4 +1,5 @@
-// Host-side interface of the single-pass index kernel (index_kernel.cu).
+// Host-side interface of the index kernels (index_tiles.cu, index_lines.cu,
+// index_exact.cu) and the newline index (newline_index.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -31,7 +32,6 @@ struct TileFile {
     uint64_t* newline_bits;
     unsigned long long* status;  // [0] line count, [1] error bits
     int64_t tile_begin;
-    uint64_t* colon;          // line-parallel kernel, optional: ':' outside strings
     // standalone kernel, optional (both or none): see IndexParams
     uint64_t* marks;
     uint32_t* odd;
@@ -65,8 +65,6 @@ struct IndexParams {
     // the newline count of every tile, in place of the newline index.
     uint64_t* newline_bits;
     int32_t* tile_newlines;
-    // Optional: the ':' bytes outside strings (ceil(n/64) words).
-    uint64_t* colon;
     // Standalone kernel, optional, what find_value's key searches jump by:
     // `marks` (ceil(n/64) words): the ':' outside strings and the quotes that
     // open a string; `odd`, one bit per word of 64 bytes (32 words to an

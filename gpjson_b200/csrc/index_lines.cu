@@ -215,7 +215,7 @@ struct FShared {
     uint8_t bytes[kByteSlots][kSlotBytes];
     TileFile desc[kRing];  // the file of the tile (by tile number modulo kRing)
     uint64_t str[kMaskSlots][kSlotWords];
-    // (read four words at a time by the interpreter)
+    // (read in pairs of words by the interpreter)
     alignas(32) uint64_t colon[kMaskSlots][kSlotWords];
     alignas(32) uint64_t lv[kMaskSlots][LV][kSlotWords];
     uint64_t nlmask[kMaskSlots][kTileWords];
@@ -527,7 +527,6 @@ __device__ __forceinline__ void finish_word(const IndexParams& p, const TileFile
     }
     if (owned && p.materialize) {
         F.string_index[word] = in_str;
-        if (F.colon) F.colon[word] = m.colon & ~in_str;
 #pragma unroll
         for (int l = 0; l < LV; l++)
             if (l < p.num_levels) F.leveled[F.level_size * l + word] = lv[l];

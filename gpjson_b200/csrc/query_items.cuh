@@ -58,7 +58,9 @@ GPJ_HD bool query_by_warp(int64_t lines, int64_t bytes, int num_queries, int64_t
 }
 
 // Mean line length under which a thread reads one bitmap word at a time
-// (Words, interp.cuh: a line of under four words rarely wants the next).
+// (Words, interp.cuh: a line of under four words rarely wants the next).  Only
+// for a whole file: the files of a batch's launch differ in their lines, and a
+// chunk's lines are not counted when its queries are launched.
 constexpr int64_t kShortLineBytes = 256;
 
 }  // namespace gpj

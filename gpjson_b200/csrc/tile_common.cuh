@@ -65,12 +65,6 @@ __device__ __forceinline__ void restrict_masks(ClassMasks& m, uint64_t keep) {
     m.colon &= keep;
 }
 
-// Escape state of the first byte of word w (parity of the backslash run that
-// ends just before it).  Taken from the previous word's trailing run through
-// a shuffle; the first lane of a warp, or a word after an all-backslash
-// word, scans the bytes before it in shared memory down to `floor` (a byte
-// index in buf) and adds `parity_at_floor` (the escape state of byte floor)
-// when the run reaches it.  Must be called by all 32 lanes.
 // Escape state of byte 64w from the bytes before it in buf: parity of the
 // backslash run ending at byte 64w - 1, scanned down to `floor` (plus
 // `parity_at_floor` when the run reaches it).
@@ -85,6 +79,12 @@ __device__ __forceinline__ uint32_t escape_scan_back(const uint8_t* buf, int w, 
     return static_cast<uint32_t>(c);
 }
 
+// Escape state of the first byte of word w (parity of the backslash run that
+// ends just before it).  Taken from the previous word's trailing run through
+// a shuffle; the first lane of a warp, or a word after an all-backslash
+// word, scans the bytes before it in shared memory down to `floor` (a byte
+// index in buf) and adds `parity_at_floor` (the escape state of byte floor)
+// when the run reaches it.  Must be called by all 32 lanes.
 __device__ __forceinline__ uint32_t escape_carry_in(const uint8_t* buf, int w, uint64_t backslash, int floor,
                                                     int parity_at_floor) {
     const int lane = threadIdx.x & 31;
@@ -99,65 +99,6 @@ __device__ __forceinline__ uint32_t escape_carry_in(const uint8_t* buf, int w, u
 __device__ __forceinline__ Span shfl_span_up(const Span& v, int off) {
     return Span{__shfl_up_sync(~0u, v.q, off), __shfl_up_sync(~0u, v.dd0, off), __shfl_up_sync(~0u, v.ddt, off),
                 __shfl_up_sync(~0u, v.nl, off)};
-}
-
-// Exclusive compose-scan of one Span per thread across the CTA, in thread
-// order.  `scratch` holds kTileWarps Spans.  Contains one __syncthreads; the
-// caller must barrier before `scratch` is reused.
-__device__ __forceinline__ Span block_scan_span(Span mine, Span* scratch, Span* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    Span incl = mine;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const Span o = shfl_span_up(incl, off);
-        if (lane >= off) incl = span_compose(o, incl);
-    }
-    if (lane == 31) scratch[warp] = incl;
-    Span excl = shfl_span_up(incl, 1);
-    if (lane == 0) excl = span_identity();
-    __syncthreads();
-    Span prefix = span_identity();
-    Span all = span_identity();
-#pragma unroll
-    for (int w = 0; w < kTileWarps; w++) {
-        if (w == warp) prefix = all;
-        all = span_compose(all, scratch[w]);
-    }
-    *total = all;
-    return span_compose(prefix, excl);
-}
-
-// Exclusive sum of an int and minimum of an int64 across the CTA.  One
-// __syncthreads; `isum` holds kTileWarps ints, `imin` kTileWarps int64.
-__device__ __forceinline__ int block_sum_min(int x, int64_t y, int* isum, int64_t* imin, int* total,
-                                             int64_t* minimum) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = x;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int o = __shfl_up_sync(~0u, incl, off);
-        if (lane >= off) incl += o;
-    }
-    int64_t mn = y;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const int64_t o = __shfl_xor_sync(~0u, mn, off);
-        mn = o < mn ? o : mn;
-    }
-    if (lane == 31) isum[warp] = incl;
-    if (lane == 0) imin[warp] = mn;
-    __syncthreads();
-    int before = 0, all = 0;
-    int64_t m = imin[0];
-#pragma unroll
-    for (int w = 0; w < kTileWarps; w++) {
-        if (w < warp) before += isum[w];
-        all += isum[w];
-        m = imin[w] < m ? imin[w] : m;
-    }
-    *total = all;
-    *minimum = m;
-    return before + incl - x;
 }
 
 // Issues the TMA load of [start, start + bytes) into `dst` on `bar` (one thread).
@@ -180,7 +121,7 @@ __device__ __forceinline__ void load_slot(const uint8_t* file, int64_t start, in
 __device__ __forceinline__ void fetch_tile_file(const IndexParams& p, int64_t t, TileFile* out) {
     if (p.batch_files == 0) {
         *out = TileFile{p.file,     p.n,     p.avail,        p.string_index, p.leveled,
-                        p.level_size, p.newline_bits, p.status, 0, p.colon, p.marks, p.odd};
+                        p.level_size, p.newline_bits, p.status, 0, p.marks, p.odd};
         return;
     }
     int lo = 0, hi = p.batch_files - 1;  // last file with tile_begin <= t

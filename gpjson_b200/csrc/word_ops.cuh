@@ -69,14 +69,6 @@ GPJ_HD int clz64(uint64_t x) {  // x != 0
 #endif
 }
 
-GPJ_HD uint32_t mulhi32(uint32_t a, uint32_t b) {
-#ifdef __CUDA_ARCH__
-    return __umulhi(a, b);
-#else
-    return static_cast<uint32_t>((static_cast<uint64_t>(a) * b) >> 32);
-#endif
-}
-
 // 0x80 in every byte of x equal to the byte replicated in `pattern`
 // (pattern bytes < 0x80), 0 elsewhere.  Exact for all 256 byte values:
 // the low seven bits are compared with a carry-free add, bit 7 must be 0.
