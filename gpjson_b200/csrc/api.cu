@@ -442,7 +442,8 @@ int ensure_tile_state(gpj_ctx* ctx, int64_t ntiles) {
         // next file's from the place of the last one's, and the pool remaps
         // memory for them at every load (2 GiB with little to spare: 41.3 ms
         // a load, now and then 50 to 1000, instead of 40.7)
-        const int64_t cap = std::max<int64_t>({words, 3 * 4096, ctx->tile_state_words * 3 / 2});
+        // (for 1 GiB of input from the start: 2 MiB is what it takes anyway)
+        const int64_t cap = std::max<int64_t>({words, 3 << 16, ctx->tile_state_words * 3 / 2});
         GPJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         if (ctx->d_tile_state) cudaFree(ctx->d_tile_state);
         ctx->d_tile_state = nullptr;
