@@ -96,6 +96,7 @@ struct __align__(128) Shared {
     // per warp: level change (low 16 bits, signed) + newlines << 16
     int32_t change[2][kWarps];
     int32_t first[2];  // level change from the start of the first '\n''s warp up to it
+    alignas(8) uint8_t passes[kWarps];  // the warp's words are backslashes alone
     // the look-back's sums and result
     int32_t dd0[kWarps], ddt[kWarps];
     int32_t s0;
@@ -152,7 +153,7 @@ __device__ __forceinline__ int first_answer(int mine) {
 // tile (a build with one run of 33 MiB 2.9 ms, of 512 MiB 45 ms; of as many
 // other bytes 0.07 and 0.5 ms).  Each word for itself walking back to the
 // run's first byte costs the square of its length.
-__device__ __noinline__ uint32_t escape_before(Shared& sh, int b, int w) {
+__device__ __forceinline__ uint32_t parity_before(Shared& sh, int b, int w) {
     const int lane = threadIdx.x & 31;
     const uint8_t* const bytes = tile_bytes(sh);
     const int64_t tile_start = (sh.tile[b] - sh.desc[b].tile_begin) * kTile;
@@ -191,6 +192,14 @@ __device__ __noinline__ uint32_t escape_before(Shared& sh, int b, int w) {
         }
         __nanosleep(64);
     }
+}
+
+// The same, out of line (inline it costs the kernel registers); the tile's first
+// byte's is kept for the tile after it.
+__device__ __noinline__ uint32_t escape_before(Shared& sh, int b, int w) {
+    const uint32_t e = parity_before(sh, b, w);
+    if (threadIdx.x == 0) sh.escape = e;
+    return e;
 }
 
 // State before tile t of a file whose first tile is t0 (one warp): the tiles
@@ -336,10 +345,7 @@ __global__ void __launch_bounds__(kThreads, LV <= 8 ? 6 : 5) tile_index_kernel(I
             ballot_b = __ballot_sync(~0u, bs != 0);
             const int first = 64 * 32 * warp;
             uint32_t cin = 0;  // of the warp's first byte
-            if ((warp > 0 || tile_start > 0) && bytes[first - 1] == '\\') {
-                cin = escape_before(sh, b, first);
-                if (tid == 0) sh.escape = cin;
-            }
+            if ((warp > 0 || tile_start > 0) && bytes[first - 1] == '\\') cin = escape_before(sh, b, first);
             if (ballot_b) {
                 // (a word of backslashes passes on what it was given)
                 const unsigned runs = __ballot_sync(~0u, trailing_run_odd(bs));
@@ -377,20 +383,23 @@ __global__ void __launch_bounds__(kThreads, LV <= 8 ? 6 : 5) tile_index_kernel(I
                 const uint64_t outside = ~(p0 ^ (s_warp ? ~0ull : 0ull));
                 const int dd0 = __reduce_add_sync(~0u, popc64(open & outside) - popc64(close & outside));
                 const int ddt = __reduce_add_sync(~0u, popc64(open) - popc64(close));
-                if (lane == 0) {
-                    sh.dd0[warp] = dd0;
-                    sh.ddt[warp] = ddt;
-                }
                 // a tile of backslashes alone (its words still lie in the slot)
                 bool passes = ballot_b == ~0u && !tail;
                 if (passes) {
 #pragma unroll
                     for (int i = 0; i < 4; i++)
                         passes = passes && run_at_end(*reinterpret_cast<const uint4*>(bytes + 64 * tid + 16 * i)) < 0;
+                    passes = __all_sync(~0u, passes);
                 }
-                const bool all_pass = __syncthreads_and(passes);
+                if (lane == 0) {
+                    sh.dd0[warp] = dd0;
+                    sh.ddt[warp] = ddt;
+                    sh.passes[warp] = passes ? 1 : 0;
+                }
+                __syncthreads();
                 if (warp == 0) {
                     if (lane == 0) {
+                        const bool all_pass = *reinterpret_cast<const uint64_t*>(sh.passes) == 0x0101010101010101ull;
                         const unsigned long long escape = all_pass && bytes[-1] == '\\' ? sh.escape : 0;
                         int e0 = 0, et = 0;
 #pragma unroll
