@@ -31,14 +31,14 @@
 // summaries), and after their level changes (one shuffle scan).  The level
 // split is bit-parallel (split_half), so no lane waits for a denser word.
 //
-// Bound by integer operations: the ALU pipe is 83 % busy at 256 MiB of tweets
-// (128 us, DRAM bytes = input + index, 0.41 warp instructions per byte),
+// Bound by integer operations: the ALU pipe is 84 % busy at 256 MiB of tweets
+// (128 us, DRAM bytes = input + index, 0.40 warp instructions per byte),
 // DRAM at 43 % of its rate.  The kernel this one replaced (30 KiB tiles
 // with a 2 KiB look-ahead each, word state kept in shared memory between two
 // passes, the level split dealt over the warp by cuts) took 193 us there.
 // Index builds: 2 GiB of tweets 1558 -> 1076 us; 1 GiB with lines up to 1 MiB,
 // which went to the exact kernel before, 1287 -> 833 us; 256 MiB of it at 16
-// levels 900 -> 262 us; 256 MiB of 117-byte lines 269 -> 166 us.
+// levels 900 -> 263 us; 256 MiB of 117-byte lines 269 -> 166 us.
 #include <cstdint>
 
 #include "device_common.cuh"
@@ -150,7 +150,7 @@ __device__ __forceinline__ int first_answer(int mine) {
 // tile before that is backslashes throughout passes on the state of its own
 // first byte, which it publishes with its effect, so a run of any length costs
 // each of its tiles one such look and one wait: bound by that chain, 1.4 us a
-// tile (a build with one run of 33 MiB 2.9 ms, of 512 MiB 45 ms; of as many
+// tile (a build with one run of 33 MiB 3.0 ms, of 512 MiB 47 ms; of as many
 // other bytes 0.07 and 0.5 ms).  Each word for itself walking back to the
 // run's first byte costs the square of its length.
 __device__ __forceinline__ uint32_t parity_before(Shared& sh, int b, int w) {
